@@ -47,6 +47,38 @@ int aaac_build(const ufe_base_mesh *b, ufe_aaac_mesh *o, std::string *msg);
 // ufe_mesh_create with a chosen number of spatial patches (0: the single-solve default).
 int mesh_create(const ufe_mesh_desc *d, int n_patch, ufe_mesh_h *out);
 
+#ifdef __CUDACC__
+#define UFE_HD __host__ __device__ __forceinline__
+#else
+#define UFE_HD inline
+#endif
+constexpr unsigned kNoCol = 0xffffu;   // no neighbour (16-bit columns of the halo program)
+constexpr int kXchBufs = 3;     // exchange buffers, taken in turn by sweep
+
+// A halo program slice's block: eight 16-bit columns per 16-byte piece, then the coefficients
+// (mixed: two float2 per piece; FP64: one double2), then per slot the packed row word (local row,
+// 0xffff: padding; export number << 16, 0xffff: not exported) and the cross-term coefficient,
+// then the row data that change between linear solves (halo_refresh). Boundary slices (edge rows,
+// corners) have no coefficients.
+struct SliceLayout {
+  int coef, row, dat, size;   // byte offsets; the columns come first
+};
+template <bool kM>
+UFE_HD SliceLayout slice_layout(int w, bool boundary) {
+  SliceLayout s;
+  s.coef = (w > 8 ? (w + 7) / 8 : 1) * 512;
+  if (kM) {
+    s.row = s.coef + (boundary ? 0 : (w > 6 ? (w + 1) / 2 : 3) * 512);   // at least six entries are read
+    s.dat = s.row + 256;           // (local row word, 3 sNxy in FP32)
+    s.size = s.dat + 512;          // (1/eu, 1/ev, defect) or (c0 x, c0 y, 1 / count, 0)
+  } else {
+    s.row = s.coef + (boundary ? 0 : w * 512);
+    s.dat = s.row + 512;           // (local row word, 0, cross-term coefficient)
+    s.size = s.dat + (boundary ? 0 : 1536);   // fast: 1/e, RHS, -; exact: e, RHS, 1/e
+  }
+  return s;
+}
+
 // Device re-layout of the combined AaAc mesh.
 //
 // Rows are cut into spatially compact patches (Morton order of the row coordinates), one
@@ -101,37 +133,30 @@ struct DevMesh {
   int *iAci = nullptr;          // [nV * ncm] column-major Ac ids (0-based), for map_Ac_to_Aa
   int *nC = nullptr;            // [nV]
 
-  // Halo sweep program (single solves; batched members in the mixed mode). One SOR sweep runs
-  // in seven phases: colours 1..5, then the edge rows, then the corners. A patch updates,
-  // besides its own rows, the halo
-  // rows whose updates its own rows read within the same sweep (the closure of "reads a row
-  // of an earlier phase"), with the same arithmetic, so that a whole sweep needs the
-  // neighbouring patches only once, at its start. Its working copy of the velocities
-  // (shared memory) holds its own device rows [p0, p1) at local index p - p0, then its halo
-  // rows. The program lists, per phase, slices of 32 (local row, device row) slots with
-  // their entries as local columns and coefficients, in the reference's neighbour order.
+  // Halo sweep program (ufe_halo.cuh). One SOR sweep runs in seven phases: colours 1..5, then the
+  // edge rows, then the corners. A patch updates, besides its own rows, the halo rows whose
+  // updates its own rows read within the same sweep (the closure of "reads a row of an earlier
+  // phase"), with the same arithmetic, so that a whole sweep needs the neighbouring patches only
+  // once, at its start. Its working copy of the velocities (shared memory) holds its own device
+  // rows [p0, p1) at local index p - p0, then its halo rows. The program lists, per phase, slices
+  // of 32 slots, one block of columns, coefficients and row data per slice (SliceLayout), in the
+  // reference's neighbour order.
   bool has_halo = false;
   int max_local = 0;            // largest own slots + halo rows of a patch
   int max_halo = 0;             // largest number of halo rows of a patch
   int max_hslices = 0;          // largest number of program slices of a patch
-  int max_hsync = 0;
   int n_hslices = 0;
-  int64_t n_hE = 0;
+  int n_export = 0;             // rows that are another patch's halo rows
   int *hp_slice = nullptr;      // [n_patch * 7 + 1] first program slice of phases 0..6 of each patch, then the end
   int *hp_split = nullptr;      // [n_patch] first slice of phase 0's rows that read halo slots (the others come first)
-  int *hslice_e0 = nullptr;     // [n_hslices] first entry of a program slice
   uint8_t *hslice_w = nullptr;  // [n_hslices] entries per slot
-  int *hrow_l = nullptr;        // [n_hslices * 32] local row, -1 = padding
-  int *hrow_g = nullptr;        // [n_hslices * 32] device row
-  uint16_t *hcol = nullptr;     // [n_hE] local column, 0xffff = padding
-  float2 *hcuv32 = nullptr;     // [n_hE]
-  double2 *hcuv = nullptr;      // [n_hE]
-  int *hload_ptr = nullptr;     // [n_patch + 1] a patch's halo rows in hload_dev
+  int *hslice_b32 = nullptr, *hslice_b64 = nullptr;        // [n_hslices] a slice's block, in 16-byte units
+  unsigned char *hprog32 = nullptr, *hprog64 = nullptr;    // the blocks of the mixed and of the FP64 sweeps
+  int *hrow_g = nullptr;        // [n_hslices * 32] device row, -1 = padding
+  int *hload_ptr = nullptr;     // [n_patch + 1] a patch's halo rows in hload_dev, hload_ex
   int *hload_dev = nullptr;     // device row of each halo slot
-  int *hsync_ptr = nullptr;     // [n_patch + 1] patches a patch waits for / is waited for by
-  int *hsync_list = nullptr;
-  float *hs3_32 = nullptr;      // [n_hslices * 32] 3 sNxy of the slot's row (FP32), 0 on padding
-  double *hs3 = nullptr;        // [n_hslices * 32] the same in FP64
+  int *hload_ex = nullptr;      // its number among the exported rows
+  int *hex_ptr = nullptr;       // [n_patch + 1] a patch's exported rows
 };
 
 struct SsaWork;   // per-handle device buffers of the SSA solve (ufe_ssa.cu)

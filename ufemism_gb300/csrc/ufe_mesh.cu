@@ -57,9 +57,9 @@ void free_mesh(DevMesh &m) {
   void *ptrs[] = {m.orig_of_dev, m.dev_of_orig, m.deg, m.slice_ptr, m.col, m.cuv, m.nxy,
                   m.cuv32, m.nxy32, m.h_nxy, m.h_cuv, m.sNxy, m.s3Nxy, m.h_nxy32, m.s3Nxy32, m.bnd_ptr,
                   m.bnd_nbr, m.V, m.Aci12, m.iAci, m.nC, m.patch_slice, m.patch_edge0, m.edge_row,
-                  m.sync_ptr, m.sync_list, m.slice_e0, m.slice_w, m.slice_g, m.hp_slice, m.hp_split, m.hslice_e0,
-                  m.hslice_w, m.hrow_l, m.hrow_g, m.hcol, m.hcuv32, m.hcuv, m.hload_ptr, m.hload_dev,
-                  m.hsync_ptr, m.hsync_list, m.hs3_32, m.hs3};
+                  m.sync_ptr, m.sync_list, m.slice_e0, m.slice_w, m.slice_g, m.hp_slice, m.hp_split, m.hslice_w,
+                  m.hslice_b32, m.hslice_b64, m.hprog32, m.hprog64, m.hrow_g, m.hload_ptr, m.hload_dev, m.hload_ex,
+                  m.hex_ptr};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   m = DevMesh();
@@ -395,18 +395,21 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
   m.max_sync = max_sync;
   if (max_sync > kMaxSync) { set_error("ufe_mesh_create: a patch touches too many other patches"); return UFE_BAD_MESH; }
 
-  // ---- halo sweep program (single solves only) --------------------------------------------
+  // ---- halo sweep program -----------------------------------------------------------------
   // Phases of a sweep: colours 0..4 (non-edge rows), 5 edge rows, 6 corners; an update reads
   // CAaAc neighbours (edge rows: the non-edge ones). A patch must also update every row of an
   // earlier phase that one of its updates reads (transitively): such a row is current only
   // after its own update in this sweep. Everything else it reads is a start-of-sweep value.
   std::vector<int> hp_slice, hp_split, hslice_e0, hrow_l, hrow_g, hload_ptr(1, 0), hload_dev, hsync_ptr(1, 0), hsync_list;
+  std::vector<int> hex_ptr(n_patch + 1, 0), hload_ex;
   std::vector<uint8_t> hslice_w;
   std::vector<uint16_t> hcol;
   std::vector<float2> hcuv32;
   std::vector<double2> hcuv;
+  std::vector<int> hslice_b32, hslice_b64;        // first 16-byte unit of each slice's block
+  std::vector<unsigned char> hprog32, hprog64;    // the blocks (SliceLayout)
   bool halo_ok = true;
-  if (halo_ok) {
+  {
     std::vector<int8_t> ph(m.nP, -1);
     for (int p = 0; p < m.nP; ++p) {
       const int r = orig_of_dev[p];
@@ -422,12 +425,13 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
       }
     };
     std::vector<int> in_r(m.nP, -1), lidx(m.nP, -1), stamp(m.nP, -1), rd;
-    std::vector<std::vector<int>> hreads(n_patch);
-    int64_t nE_h = 0;
+    std::vector<std::vector<int>> hreads(n_patch), upd(n_patch);
+    // every patch's updated rows and halo rows (each row read or updated that is not its own), the
+    // halo in device-row order: a reader's loads of one owner's exported rows are then contiguous
     for (int b = 0; b < n_patch && halo_ok; ++b) {
       const int p0 = patch_slice[(size_t)b * (kGroups + 1)] * kSlice;
       const int p1 = patch_slice[(size_t)b * (kGroups + 1) + kGroups] * kSlice;
-      std::vector<int> R;
+      std::vector<int> &R = upd[b];
       for (int p = p0; p < p1; ++p)
         if (ph[p] >= 0) { in_r[p] = b; R.push_back(p); }
       for (size_t k = 0; k < R.size(); ++k) {
@@ -435,25 +439,51 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
         for (int j : rd)
           if (ph[j] < ph[R[k]] && in_r[j] != b) { in_r[j] = b; R.push_back(j); }
       }
-      // local slots: own device rows first, then the halo rows (every row read or updated)
-      const int n_own = p1 - p0;
       std::vector<int> halo;
-      auto local_of = [&](int p) {
-        if (p >= p0 && p < p1) return p - p0;
-        if (stamp[p] != b) { stamp[p] = b; lidx[p] = n_own + (int)halo.size(); halo.push_back(p); }
-        return lidx[p];
+      auto see = [&](int p) {
+        if ((p >= p0 && p < p1) || stamp[p] == b) return;
+        stamp[p] = b;
+        halo.push_back(p);
       };
       for (int p : R) {
-        local_of(p);
+        see(p);
         reads_of(p, rd);
-        for (int j : rd) local_of(j);
+        for (int j : rd) see(j);
       }
-      if (n_own + (int)halo.size() > 65535) { halo_ok = false; break; }
+      std::sort(halo.begin(), halo.end());
+      const int n_own = p1 - p0;
+      if (n_own + (int)halo.size() > 65533) { halo_ok = false; break; }
       m.max_local = std::max(m.max_local, n_own + (int)halo.size());
       m.max_halo = std::max(m.max_halo, (int)halo.size());
       for (int p : halo) hreads[b].push_back(patch_of[orig_of_dev[p]]);
       hload_dev.insert(hload_dev.end(), halo.begin(), halo.end());
       hload_ptr.push_back((int)hload_dev.size());
+    }
+    // exported rows (halo rows of some other patch), numbered in device-row order: a patch's are
+    // [hex_ptr[b], hex_ptr[b + 1])
+    std::vector<int> export_of(m.nP, -1);
+    if (halo_ok) {
+      for (int p : hload_dev) export_of[p] = 0;
+      int n = 0;
+      for (int b = 0; b < n_patch; ++b) {
+        hex_ptr[b] = n;
+        for (int p = patch_slice[(size_t)b * (kGroups + 1)] * kSlice;
+             p < patch_slice[(size_t)b * (kGroups + 1) + kGroups] * kSlice; ++p)
+          if (export_of[p] == 0) export_of[p] = n++;
+      }
+      hex_ptr[n_patch] = n;
+      m.n_export = n;
+      hload_ex.reserve(hload_dev.size());
+      for (int p : hload_dev) hload_ex.push_back(export_of[p]);
+    }
+    int64_t nE_h = 0;
+    for (int b = 0; b < n_patch && halo_ok; ++b) {
+      const int p0 = patch_slice[(size_t)b * (kGroups + 1)] * kSlice;
+      const int p1 = patch_slice[(size_t)b * (kGroups + 1) + kGroups] * kSlice;
+      const int n_own = p1 - p0;
+      const std::vector<int> &R = upd[b];
+      for (int i = hload_ptr[b]; i < hload_ptr[b + 1]; ++i) lidx[hload_dev[i]] = n_own + i - hload_ptr[b];
+      auto local_of = [&](int p) { return p >= p0 && p < p1 ? p - p0 : lidx[p]; };
       // program: per phase, the phase's own and halo rows packed densely into slices of 32
       // (bank_aware_slices: by degree, lanes chosen to spread the working-copy gathers over
       // the shared-memory banks)
@@ -501,25 +531,55 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
           }
           hslice_e0.push_back((int)nE_h);
           hslice_w.push_back((uint8_t)w);
-          hcol.resize((size_t)nE_h + (size_t)w * kSlice, 0xffff);
-          hcuv32.resize((size_t)nE_h + (size_t)w * kSlice, make_float2(0, 0));
-          hcuv.resize((size_t)nE_h + (size_t)w * kSlice, make_double2(0, 0));
+          if (t_dump_path) {
+            hcol.resize((size_t)nE_h + (size_t)w * kSlice, 0xffff);
+            hcuv32.resize((size_t)nE_h + (size_t)w * kSlice, make_float2(0, 0));
+            hcuv.resize((size_t)nE_h + (size_t)w * kSlice, make_double2(0, 0));
+          }
+          const SliceLayout y32 = slice_layout<true>(w, f >= 5), y64 = slice_layout<false>(w, f >= 5);
+          const size_t o32 = hprog32.size(), o64 = hprog64.size();
+          hslice_b32.push_back((int)(o32 / 16));
+          hslice_b64.push_back((int)(o64 / 16));
+          hprog32.resize(o32 + y32.size, 0);
+          hprog64.resize(o64 + y64.size, 0);
+          unsigned char *q32 = hprog32.data() + o32, *q64 = hprog64.data() + o64;
+          std::memset(q32, 0xff, y32.coef);   // no column
+          std::memset(q64, 0xff, y64.coef);
+          if (f < 5)   // mixed colour slices: missing entries name the working copy's zero slot
+            for (int i = 0; i < y32.coef / 2; ++i) reinterpret_cast<uint16_t *>(q32)[i] = (uint16_t)(n_own + hload_ptr[b + 1] - hload_ptr[b]);
           for (int l = 0; l < kSlice; ++l) {
             const int p = rows[s0 + l];
-            hrow_l.push_back(p < 0 ? -1 : local_of(p));
+            const int loc = p < 0 ? -1 : local_of(p);
+            hrow_l.push_back(loc);
             hrow_g.push_back(p < 0 ? 0 : p);
+            // the packed row word: the export number counts from the patch's first
+            const unsigned ex = p >= p0 && p < p1 && export_of[p] >= 0 ? (unsigned)(export_of[p] - hex_ptr[b]) : kNoCol;
+            const unsigned word = p < 0 ? 0xffffffffu : (ex << 16) | (unsigned)loc;
+            std::memcpy(q32 + y32.row + l * 8, &word, 4);
+            std::memcpy(q64 + y64.row + l * 16, &word, 4);
             if (p < 0) continue;
+            std::memcpy(q32 + y32.row + l * 8 + 4, &s3Nxy32[p], 4);
+            std::memcpy(q64 + y64.row + l * 16 + 8, &s3Nxy[p], 8);
             reads_of(p, rd);
             // the device SELL entries of p hold the same neighbours in the same order (the
             // edge rows' list skips their edge neighbours: their coefficients are unused)
             const int s = p / kSlice, ln = p % kSlice;
             for (size_t k = 0; k < rd.size(); ++k) {
               const size_t e = (size_t)nE_h + k * kSlice + l;
-              hcol[e] = (uint16_t)local_of(rd[k]);
+              const int64_t ed = slice_ptr[s] + (int64_t)k * kSlice + ln;
+              const uint16_t c16 = (uint16_t)local_of(rd[k]);
+              std::memcpy(q32 + (k / 8) * 512 + l * 16 + (k % 8) * 2, &c16, 2);
+              std::memcpy(q64 + (k / 8) * 512 + l * 16 + (k % 8) * 2, &c16, 2);
               if (f < 5) {
-                const int64_t ed = slice_ptr[s] + (int64_t)k * kSlice + ln;
-                hcuv32[e] = cuv32[ed];
-                hcuv[e] = cuv[ed];
+                std::memcpy(q32 + y32.coef + (k / 2) * 512 + l * 16 + (k % 2) * 8, &cuv32[ed], 8);
+                std::memcpy(q64 + y64.coef + k * 512 + l * 16, &cuv[ed], 16);
+              }
+              if (t_dump_path) {
+                hcol[e] = c16;
+                if (f < 5) {
+                  hcuv32[e] = cuv32[ed];
+                  hcuv[e] = cuv[ed];
+                }
               }
             }
           }
@@ -527,11 +587,12 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
         }
       }
       m.max_hslices = std::max(m.max_hslices, (int)hslice_e0.size() - first_slice);
-      if (m.max_hslices > kMaxPatchSlices || nE_h >= ((int64_t)1 << 31)) halo_ok = false;
+      if (m.max_hslices > kMaxPatchSlices || nE_h >= ((int64_t)1 << 31) ||
+          hprog64.size() / 16 >= ((size_t)1 << 31)) halo_ok = false;
     }
     if (halo_ok) {
       hp_slice.push_back((int)hslice_e0.size());   // end of the last patch
-      // the start-of-sweep wait: the owners of a patch's halo rows, and the patches that read it
+      // the patches that exchange rows (symmetric closure; a check of the layout's consistency)
       std::vector<std::vector<int>> hs(n_patch);
       for (int b = 0; b < n_patch; ++b)
         for (int q : hreads[b])
@@ -539,13 +600,10 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
       for (int b = 0; b < n_patch; ++b) {
         std::sort(hs[b].begin(), hs[b].end());
         hs[b].erase(std::unique(hs[b].begin(), hs[b].end()), hs[b].end());
-        m.max_hsync = std::max(m.max_hsync, (int)hs[b].size());
         hsync_list.insert(hsync_list.end(), hs[b].begin(), hs[b].end());
         hsync_ptr.push_back((int)hsync_list.size());
       }
-      if (m.max_hsync > kMaxSync) halo_ok = false;
       m.n_hslices = (int)hslice_e0.size();
-      m.n_hE = nE_h;
     }
   }
   m.has_halo = halo_ok;
@@ -584,6 +642,8 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
     f.put("hrow_l", hrow_l); f.put("hrow_g", hrow_g); f.put("hcol", hcol); f.put("hcuv", hcuv);
     f.put("hcuv32", hcuv32); f.put("hload_ptr", hload_ptr); f.put("hload_dev", hload_dev);
     f.put("hsync_ptr", hsync_ptr); f.put("hsync_list", hsync_list);
+    f.put("hslice_b32", hslice_b32); f.put("hprog32", hprog32); f.put("hslice_b64", hslice_b64); f.put("hprog64", hprog64);
+    f.put("hload_ex", hload_ex); f.put("hex_ptr", hex_ptr);
     return f.ok() ? UFE_OK : UFE_BAD_ARG;
   }
 
@@ -625,25 +685,18 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
   if (!rc && m.has_halo) {
     rc = upload(&m.hp_slice, hp_slice, S, "hp_slice");
     if (!rc) rc = upload(&m.hp_split, hp_split, S, "hp_split");
-    if (!rc) rc = upload(&m.hslice_e0, hslice_e0, S, "hslice_e0");
     if (!rc) rc = upload(&m.hslice_w, hslice_w, S, "hslice_w");
-    if (!rc) rc = upload(&m.hrow_l, hrow_l, S, "hrow_l");
+    if (!rc) rc = upload(&m.hslice_b32, hslice_b32, S, "hslice_b32");
+    if (!rc) rc = upload(&m.hslice_b64, hslice_b64, S, "hslice_b64");
+    if (!rc) rc = upload(&m.hprog32, hprog32, S, "hprog32");
+    if (!rc) rc = upload(&m.hprog64, hprog64, S, "hprog64");
+    for (size_t k = 0; k < hrow_g.size(); ++k)
+      if (hrow_l[k] < 0) hrow_g[k] = -1;
     if (!rc) rc = upload(&m.hrow_g, hrow_g, S, "hrow_g");
-    if (!rc) rc = upload(&m.hcol, hcol, S, "hcol");
-    if (!rc) rc = upload(&m.hcuv32, hcuv32, S, "hcuv32");
-    if (!rc) rc = upload(&m.hcuv, hcuv, S, "hcuv");
     if (!rc) rc = upload(&m.hload_ptr, hload_ptr, S, "hload_ptr");
     if (!rc) rc = upload(&m.hload_dev, hload_dev, S, "hload_dev");
-    if (!rc) rc = upload(&m.hsync_ptr, hsync_ptr, S, "hsync_ptr");
-    if (!rc) rc = upload(&m.hsync_list, hsync_list, S, "hsync_list");
-    // per-slot copies of the static cross-term coefficient (the kernels then need no
-    // dependent load through the slot's device row)
-    std::vector<float> hs3_32(hrow_g.size(), 0.0f);
-    std::vector<double> hs3(hrow_g.size(), 0.0);
-    for (size_t k = 0; k < hrow_g.size(); ++k)
-      if (hrow_l[k] >= 0) { hs3_32[k] = s3Nxy32[hrow_g[k]]; hs3[k] = s3Nxy[hrow_g[k]]; }
-    if (!rc) rc = upload(&m.hs3_32, hs3_32, S, "hs3_32");
-    if (!rc) rc = upload(&m.hs3, hs3, S, "hs3");
+    if (!rc) rc = upload(&m.hload_ex, hload_ex, S, "hload_ex");
+    if (!rc) rc = upload(&m.hex_ptr, hex_ptr, S, "hex_ptr");
   }
   if (!rc) rc = cuda_status(cudaStreamSynchronize(S), "mesh upload");
   h->m = m;

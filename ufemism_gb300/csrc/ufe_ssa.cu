@@ -102,20 +102,20 @@ struct SsaArgs {
   const int *edge_row;
   const int *sync_ptr;
   const int *sync_list;
-  // halo sweep program (DevMesh, ufe_internal.h)
-  const int *hp_slice, *hslice_e0;
+  // halo sweep program (DevMesh, ufe_internal.h) of the solve's precision
+  const int *hp_slice;
   const int *hp_split;     // first slice of phase 0's rows that read halo slots
+  const int *hslice_b0;    // first 16-byte unit of each slice's block in hprog
   const uint8_t *hslice_w;
-  const int *hrow_l, *hrow_g;
-  const uint16_t *hcol;
-  const float2 *hcuv32;
-  const double2 *hcuv;
-  const int *hload_ptr, *hload_dev, *hsync_ptr, *hsync_list;
-  const float *hs3_32;
-  const double *hs3;
-  float4 *hsd32;           // halo sweeps, mixed: per slot (1/eu, 1/ev, defect x, y) in FP32;
-                           // boundary slots: (c0 x, c0 y, 1 / count, 0), see halo_boundary
-  double2 *hrcp, *hrhs;    // halo sweeps, fast FP64: per slot (1/eu, 1/ev) and (RHSx, RHSy)
+  const int *hrow_g;
+  const int *hload_ptr, *hload_dev, *hload_ex, *hex_ptr;
+  unsigned char *hprog;
+  double2 *hundo;             // FP64: each program slot's value before its last update
+  unsigned long long *hxch;   // kXchBufs exchange buffers of xch_stride words
+  double *res_part;           // [kLagRing * CTAs] each CTA's maximum |res| by sweep
+  size_t xch_stride;
+  float tol32;                // smallest FP32 value not below tol
+  float omega32;              // omega rounded to FP32
   float4 *bc0;             // mixed, per edge ordinal: (c0 x, c0 y, 1 / count, 0), see phase_boundary
   unsigned int *prog;      // per-CTA progress counters (stride 32 words)
   int n_edge;              // edge ordinals (edge rows and corners)
@@ -127,8 +127,6 @@ struct SsaArgs {
   const uint8_t *skip;    // Dirichlet rows (grounding-line Ac rows under the GL-flux option), may be null
   double2 *UV;            // FP64 velocities (u0 in the mixed path)
   float2 *dUV;            // mixed: correction d
-  double2 *UVb, *UVc;     // halo sweeps, FP64 modes: the second and third velocity buffers
-  float2 *dUVb, *dUVc;    // halo sweeps, mixed: the second and third correction buffers
   float2 *r0;             // mixed: defect
   float2 *rcp32;          // mixed: FP32 reciprocals of (eu, ev)
   double *eta, *Na, *Nb, *S;
@@ -142,7 +140,7 @@ struct SsaArgs {
   int fp32_visc;
   int local_rows;          // keep the patch's own velocities (mixed: corrections) in shared memory
   int halo_index_off;      // halo sweeps: byte offset of the halo slots' device rows in dynamic shared memory
-  int stage_off, stage_bytes;   // halo sweeps, mixed: the resident program slices' area in dynamic shared memory
+  int stage_off, stage_bytes;   // halo sweeps: the resident program slices' area in dynamic shared memory
   long long timeout_ns;
 };
 
@@ -161,13 +159,11 @@ static_assert(kMixedLag >= 0 && kMixedLag <= kMaxLag, "lag out of range");
 // Largest shared-memory mirror of a patch's rows (the rest of the 228 KB of an SM stays L1).
 constexpr size_t kLocalRowsMaxBytes = 160 * 1024;
 constexpr int kMaxKrylovRestart = 1000;   // largest GMRES restart length of the VJP
-// Threads per CTA of the halo sweeps. Measured on the 200k dome: 1024 threads, one slice per
-// warp at a time, 27.1 us per mixed sweep; 768 threads with two slices' loads issued together
-// per warp (80 registers), 28.6 us.
-#ifndef UFE_HALO_BLOCK
-#define UFE_HALO_BLOCK 1024
-#endif
-constexpr int kHaloBlock = UFE_HALO_BLOCK;
+// Threads per CTA of the halo sweeps: 128 registers hold a slice's program across a barrier. On
+// the 200k dome a mixed sweep measured 18.1 us with 1024 threads (64 registers, spilled), 13.7 with
+// 512 and 18.0 with 256; at 16k vertices 8.6, 5.1 and 5.0 (before the row updates were shortened,
+// which left 12.1 and 4.3 at 512).
+constexpr int kHaloBlock = 512;
 
 // Per-phase timers of the persistent solver (profiling build only, -DUFE_PHASE_TIMERS=1):
 // thread 0 of every CTA stamps clock64() at the end of each phase of the SOR loop (every
@@ -479,11 +475,9 @@ __device__ void phase_coefficients(const SsaArgs &a, const Team &t) {
       c = h;
     }
     a.euv[p] = c;
-    if (kMode != kExact64) {
-      const double2 r = make_double2(1.0 / c.x, 1.0 / c.y);
-      a.rcp[p] = r;
-      if (kMode == kMixed) a.rcp32[p] = make_float2((float)r.x, (float)r.y);
-    }
+    const double2 r = make_double2(1.0 / c.x, 1.0 / c.y);
+    a.rcp[p] = r;
+    if (kMode == kMixed) a.rcp32[p] = make_float2((float)r.x, (float)r.y);
   }
 }
 
@@ -496,19 +490,9 @@ struct PatchSmem {
   int edge0, edge1;
   int nsync;
   int sync[kMaxSync];
-  // halo sweeps: program slices of the 7 phases (e0, w hold the program's slices), the own
-  // device rows [p0, p0 + n_own) and the halo slots [n_own, n_own + nh) of the working copy
-  int hps[8];
-  int hsplit;   // phase 0: slices [hps[0], hsplit) read no halo slot
-  int p0, n_own, nh, hl0;
   // lagged decisions: each slot's arrival word as this CTA last read it (lag_decide)
   unsigned long long lag_prev[8];
   int lag_act[2];
-  unsigned long long lag_pre;   // the arrival word of sweep lag_pre_g, read ahead by lag_arrive_publish
-  unsigned int lag_pre_g;
-  // halo sweeps, mixed: offset (16-byte units) of each program slice's resident copy in the
-  // staging area, -1 = read from global memory (halo_stage)
-  short soff[kMaxPatchSlices];
 };
 
 // One colour of the FP64 sweep in the reference's expression order (parity mode).
@@ -549,10 +533,7 @@ __device__ unsigned long long phase_sweep_exact(const SsaArgs &a, const PatchSme
 }
 
 constexpr int kBatch = 8;   // neighbour entries loaded in one batch (rows of higher degree load the rest)
-// halo sweeps: warps that wait for the neighbouring patches and load the halo slots while the
-// others run colour 1's halo-free rows (halo_fetch), and the loads each thread issues together
-constexpr int kFetchWarps = 4;
-constexpr int kFetchBatch = 4;
+constexpr int kFetchBatch = 4;   // halo sweeps: halo slots a thread loads together (halo_poll)
 
 // One colour of the fast FP64 sweep: res = U + ((sum + 3 sNxy V) - RHS) / eu with the
 // reciprocal of eu formed once per Picard iteration, products accumulated with FMA.
@@ -745,361 +726,6 @@ __device__ void phase_boundary(const SsaArgs &a, const PatchSmem &ps, const Loca
   }
 }
 
-// ---------------------------------------------------------------------------------------
-// Halo sweeps: one phase of the sweep program over this patch's working copy `ld` (shared
-// memory; own rows, then halo rows). Every update uses the arithmetic, and the neighbour
-// order, of the phased sweeps above, so an own row gets the same value either way; own rows
-// are also written to `out` (the buffer the neighbours read at the next sweep's start) and
-// alone enter the maximum residual.
-// ---------------------------------------------------------------------------------------
-constexpr uint16_t kNoCol = 0xffff;
-
-__device__ __forceinline__ int halo_global(const SsaArgs &a, const PatchSmem &ps, int l) {
-  return l < ps.n_own ? ps.p0 + l : a.hload_dev[ps.hl0 + l - ps.n_own];
-}
-
-// One slice of a colour phase of the FP32 correction sweep (as phase_sweep32), its entries
-// read through pointers already offset by the lane (entry k of the lane at [32 k]).
-__device__ __forceinline__ void slice32(const SsaArgs &a, const PatchSmem &ps, int w, const uint16_t *pc,
-                                        const float2 *pcu, int l, float s3, float4 sd, const int *hidx, float2 *ld,
-                                        float2 *out, float omega, float &mx) {
-  int j[kBatch];
-  float2 c[kBatch];
-#pragma unroll
-  for (int q = 0; q < kBatch; ++q) {
-    j[q] = q < w ? (int)pc[q * kSlice] : (int)kNoCol;
-    c[q] = q < w ? pcu[q * kSlice] : make_float2(0.f, 0.f);
-  }
-  if (l < 0) return;   // padding slot
-  if (a.skip && a.skip[l < ps.n_own ? ps.p0 + l : hidx[l - ps.n_own]]) return;   // a Dirichlet row
-  const float2 di = ld[l];
-  float su = 0.0f, sv = 0.0f;
-#pragma unroll
-  for (int q = 0; q < kBatch; ++q) {
-    if (j[q] != (int)kNoCol) {
-      const float2 u = ld[j[q]];
-      su = fmaf(u.x, c[q].x, su);
-      sv = fmaf(u.y, c[q].y, sv);
-    }
-  }
-  for (int k = kBatch; k < w; ++k) {
-    const int jj = pc[k * kSlice];
-    if (jj == (int)kNoCol) break;
-    const float2 cc = pcu[k * kSlice];
-    const float2 v = ld[jj];
-    su = fmaf(v.x, cc.x, su);
-    sv = fmaf(v.y, cc.y, sv);
-  }
-  const float ru = fmaf(fmaf(s3, di.y, su) - sd.z, sd.x, di.x);
-  const float rv = fmaf(fmaf(s3, di.x, sv) - sd.w, sd.y, di.y);
-  const float2 dn = make_float2(fmaf(-omega, ru, di.x), fmaf(-omega, rv, di.y));
-  ld[l] = dn;
-  if (l < ps.n_own) {
-    out[ps.p0 + l] = dn;
-    mx = fmaxf(mx, fmaxf(fabsf(ru), fabsf(rv)));
-  }
-}
-
-// Colour phase f of the FP32 correction sweep: warp w takes slices w, w + nwarps, ... (a
-// colour of a 200k-vertex patch has 42-50 slices for 32 warps). A round of 32 slices costs
-// about 0.5 us plus the time to bring its program data (about 100 KB) from L2 into the SM,
-// which is why the resident slices (halo_stage) are read from shared memory.
-__device__ unsigned long long halo_colour32(const SsaArgs &a, const PatchSmem &ps, int s_begin, int s_end, int nwarps,
-                                            const unsigned char *stage, const int *hidx, float2 *ld, float2 *out) {
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float omega = (float)a.omega;
-  float mx = 0.0f;
-  const int base = ps.hps[0];
-  for (int s = s_begin + wid; s < s_end; s += nwarps) {
-    const int w = ps.w[s - base];
-    const int so = ps.soff[s - base];
-    if (so >= 0) {
-      const unsigned char *b = stage + 16 * so;
-      const int *rl = reinterpret_cast<const int *>(b + w * kSlice * 10);
-      slice32(a, ps, w, reinterpret_cast<const uint16_t *>(b) + lane, reinterpret_cast<const float2 *>(b + w * kSlice * 2) + lane,
-              rl[lane], reinterpret_cast<const float *>(rl)[kSlice + lane], reinterpret_cast<const float4 *>(rl + 2 * kSlice)[lane],
-              hidx, ld, out, omega, mx);
-    } else {
-      const int64_t e0 = ps.e0[s - base] + lane;
-      const int slot = s * kSlice + lane;
-      slice32(a, ps, w, a.hcol + e0, a.hcuv32 + e0, a.hrow_l[slot], a.hs3_32[slot], a.hsd32[slot], hidx, ld, out, omega,
-              mx);
-    }
-  }
-  return abs_bits((double)mx);
-}
-
-// Resident program slices (mixed halo sweeps). The shared memory left after the working copy
-// and the halo indices (stage_bytes) holds, for the whole solve, copies of some of the patch's
-// colour-phase slices: the entries' local columns and coefficients, then per slot the local row,
-// 3 sNxy and the row data of halo_refresh (refreshed there with the global copy): w * 320 + 768
-// bytes for a slice of width w. Which: whole rounds (a slice per warp: 32 slices, 28 for colour
-// 1's halo-free rows, which four warps leave to the halo fetch), smallest first — the rounds after
-// the first of a colour, and whole colours of at most one round (colour 1 counting as two: its
-// halo-free rows and the others) — as many as fit. Thread 0 plans, then the CTA copies the static
-// parts.
-__device__ __forceinline__ int stage_slice_bytes(int w) { return w * kSlice * 10 + 2 * kSlice * 4 + kSlice * 16; }
-
-__device__ void halo_stage(const SsaArgs &a, PatchSmem &ps, unsigned char *stage) {
-  const int base = ps.hps[0];
-  for (int s = ps.hps[0] + (int)threadIdx.x; s < ps.hps[7]; s += blockDim.x) ps.soff[s - base] = -1;
-  __syncthreads();
-  constexpr int kMaxUnits = 40;
-  __shared__ int u0[kMaxUnits], u1[kMaxUnits], ub[kMaxUnits];
-  if (threadIdx.x == 0 && a.stage_bytes > 0) {
-    int nu = 0;
-    for (int f = -1; f < 5; ++f) {   // -1: colour 1's halo-free rows, 0: its other rows
-      const int s0 = f < 0 ? ps.hps[0] : f == 0 ? ps.hsplit : ps.hps[f];
-      const int s1 = f < 0 ? ps.hsplit : ps.hps[f + 1];
-      const int rs = (int)(blockDim.x >> 5) - (f < 0 ? kFetchWarps : 0);   // slices per round
-      for (int r = s1 - s0 <= rs ? s0 : s0 + rs; r < s1 && nu < kMaxUnits; r += rs) {
-        u0[nu] = r;
-        u1[nu] = r + rs < s1 ? r + rs : s1;
-        int b = 0;
-        for (int q = u0[nu]; q < u1[nu]; ++q) b += stage_slice_bytes(ps.w[q - base]);
-        ub[nu++] = b;
-      }
-    }
-    int used = 0;
-    for (;;) {
-      int best = -1;
-      for (int k = 0; k < nu; ++k)
-        if (ub[k] >= 0 && (best < 0 || ub[k] < ub[best])) best = k;
-      if (best < 0 || used + ub[best] > a.stage_bytes) break;
-      for (int q = u0[best]; q < u1[best]; ++q) {
-        ps.soff[q - base] = (short)(used / 16);
-        used += stage_slice_bytes(ps.w[q - base]);
-      }
-      ub[best] = -1;
-    }
-  }
-  __syncthreads();
-  const int wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5, lane = threadIdx.x & 31;
-  for (int s = ps.hps[0] + wid; s < ps.hps[5]; s += nwarps) {
-    const int so = ps.soff[s - base];
-    if (so < 0) continue;
-    unsigned char *b = stage + 16 * so;
-    const int w = ps.w[s - base];
-    const int64_t e0 = ps.e0[s - base];
-    uint16_t *pc = reinterpret_cast<uint16_t *>(b);
-    float2 *pcu = reinterpret_cast<float2 *>(b + w * kSlice * 2);
-    for (int k = lane; k < w * kSlice; k += kSlice) {
-      pc[k] = a.hcol[e0 + k];
-      pcu[k] = a.hcuv32[e0 + k];
-    }
-    int *rl = reinterpret_cast<int *>(b + w * kSlice * 10);
-    rl[lane] = a.hrow_l[s * kSlice + lane];
-    reinterpret_cast<float *>(rl)[kSlice + lane] = a.hs3_32[s * kSlice + lane];
-  }
-  __syncthreads();
-}
-
-// Colour phase f of the FP64 sweeps (as phase_sweep_exact and phase_sweep_fast).
-template <bool kExact>
-__device__ unsigned long long halo_colour64(const SsaArgs &a, const PatchSmem &ps, int s_begin, int s_end, int nwarps,
-                                            double2 *ld, double2 *out) {
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double omega = a.omega;
-  unsigned long long mx = 0ull;
-  const int base = ps.hps[0];
-  for (int s = s_begin + wid; s < s_end; s += nwarps) {
-    const int w = ps.w[s - base];
-    const int64_t e0 = ps.e0[s - base] + lane;
-    const int slot = s * kSlice + lane;
-    const int l = a.hrow_l[slot];
-    const int g = a.hrow_g[slot];
-    if (l < 0 || (a.skip && a.skip[g])) continue;
-    double su = 0.0, sv = 0.0;
-    double ru, rv;
-    const double2 ui = ld[l];
-    if (kExact) {
-      for (int k = 0; k < w; ++k) {
-        const int64_t e = e0 + (int64_t)k * kSlice;
-        const int jj = a.hcol[e];
-        if (jj == (int)kNoCol) break;
-        const double2 c = a.hcuv[e];
-        const double2 u = ld[jj];
-        su = su + u.x * c.x;
-        sv = sv + u.y * c.y;
-      }
-      const double sxy = a.sNxy[g];
-      const double Uxy = ui.x * sxy, Vxy = ui.y * sxy;
-      const double2 ec = a.euv[g];
-      const double2 b = a.rhs[g];
-      const double lhsx = (su + 3.0 * Vxy) + ec.x * ui.x;
-      const double lhsy = (sv + 3.0 * Uxy) + ec.y * ui.y;
-      ru = (lhsx - b.x) / ec.x;
-      rv = (lhsy - b.y) / ec.y;
-    } else {
-      int j[kBatch];
-#pragma unroll
-      for (int q = 0; q < kBatch; ++q) j[q] = q < w ? (int)a.hcol[e0 + (int64_t)q * kSlice] : (int)kNoCol;
-      const double s3 = a.hs3[slot];
-      const double2 r = a.hrcp[slot];
-      const double2 b = a.hrhs[slot];
-#pragma unroll
-      for (int q = 0; q < kBatch; ++q) {
-        if (j[q] != (int)kNoCol) {
-          const double2 c = a.hcuv[e0 + (int64_t)q * kSlice];
-          const double2 u = ld[j[q]];
-          su = fma(u.x, c.x, su);
-          sv = fma(u.y, c.y, sv);
-        }
-      }
-      for (int k = kBatch; k < w; ++k) {
-        const int jj = a.hcol[e0 + (int64_t)k * kSlice];
-        if (jj == (int)kNoCol) break;
-        const double2 c = a.hcuv[e0 + (int64_t)k * kSlice];
-        const double2 u = ld[jj];
-        su = fma(u.x, c.x, su);
-        sv = fma(u.y, c.y, sv);
-      }
-      ru = fma(fma(s3, ui.y, su) - b.x, r.x, ui.x);
-      rv = fma(fma(s3, ui.x, sv) - b.y, r.y, ui.y);
-    }
-    const double2 un = kExact ? make_double2(ui.x - omega * ru, ui.y - omega * rv)
-                              : make_double2(fma(-omega, ru, ui.x), fma(-omega, rv, ui.y));
-    ld[l] = un;
-    if (l < ps.n_own) {
-      out[g] = un;
-      const unsigned long long bu = abs_bits(ru), bv = abs_bits(rv);
-      mx = bu > mx ? bu : mx;
-      mx = bv > mx ? bv : mx;
-    }
-  }
-  return mx;
-}
-
-// Boundary phase f (5: edge rows, 6: corners) of apply_Neumann_boundary_AaAc: the mean of the
-// listed neighbours (edge rows: the non-edge ones; corners: all, the edge rows among them
-// already updated in phase 5), as phase_boundary. Every load of a slot is issued before any is
-// used (an edge row averages at most a few neighbours), so a phase costs one round trip.
-// Mixed: with u0 fixed between refolds, mean(u0_j + d_j) - u0_i = c0_i + mean(d_j), where
-// c0_i = mean(u0_j) - u0_i is formed in FP64 at the refresh; the sweep then adds the FP32
-// corrections only.
-template <bool kM, class T>
-__device__ void halo_boundary(const SsaArgs &a, const PatchSmem &ps, int f, T *ld, T *out) {
-  const int wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5, lane = threadIdx.x & 31;
-  const int base = ps.hps[0];
-  constexpr int kB = 4;
-  for (int s = ps.hps[f] + wid; s < ps.hps[f + 1]; s += nwarps) {
-    const int w = ps.w[s - base];
-    const int64_t e0 = ps.e0[s - base] + lane;
-    const int slot = s * kSlice + lane;
-    const int l = a.hrow_l[slot];
-    const int g = a.hrow_g[slot];
-    int jb[kB];
-#pragma unroll
-    for (int k = 0; k < kB; ++k) jb[k] = k < w ? (int)a.hcol[e0 + (int64_t)k * kSlice] : (int)kNoCol;
-    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-    if constexpr (kM) c = a.hsd32[slot];
-    if (l < 0) continue;
-    T nv;
-    if constexpr (kM) {
-      float sx = 0.0f, sy = 0.0f;
-#pragma unroll
-      for (int k = 0; k < kB; ++k)
-        if (jb[k] != (int)kNoCol) {
-          const float2 dj = ld[jb[k]];
-          sx = sx + dj.x;
-          sy = sy + dj.y;
-        }
-      for (int k = kB; k < w; ++k) {
-        const int jj = a.hcol[e0 + (int64_t)k * kSlice];
-        if (jj == (int)kNoCol) break;
-        const float2 dj = ld[jj];
-        sx = sx + dj.x;
-        sy = sy + dj.y;
-      }
-      nv = make_float2(fmaf(sx, c.z, c.x), fmaf(sy, c.z, c.y));
-    } else {
-      // the packed entries in the reference's order (padding only after the last)
-      double sx = 0.0, sy = 0.0;
-      int nvals = 0;
-#pragma unroll
-      for (int k = 0; k < kB; ++k)
-        if (jb[k] != (int)kNoCol) {
-          const double2 u = ld[jb[k]];
-          sx = sx + u.x;
-          sy = sy + u.y;
-          ++nvals;
-        }
-      for (int k = kB; k < w; ++k) {
-        const int jj = a.hcol[e0 + (int64_t)k * kSlice];
-        if (jj == (int)kNoCol) break;
-        const double2 u = ld[jj];
-        sx = sx + u.x;
-        sy = sy + u.y;
-        ++nvals;
-      }
-      if (nvals < a.ncm) { sx = sx + 0.0; sy = sy + 0.0; }
-      nv = make_double2(sx / (double)nvals, sy / (double)nvals);
-    }
-    ld[l] = nv;
-    if (l < ps.n_own) out[g] = nv;
-  }
-}
-
-// Per-slot copies of the row data a sweep reads that change between linear solves (mixed:
-// the FP32 reciprocals of the centre coefficients and the defect; fast FP64: the reciprocals
-// and the right-hand side), refreshed by each CTA for its own program slots once the
-// grid-wide phase that wrote them is complete.
-template <int kMode>
-__device__ __forceinline__ void halo_refresh(const SsaArgs &a, const PatchSmem &ps, unsigned char *stage) {
-  for (int k = 32 * ps.hps[0] + (int)threadIdx.x; k < 32 * ps.hps[7]; k += blockDim.x) {
-    if (a.hrow_l[k] < 0) continue;
-    const int g = a.hrow_g[k];
-    if constexpr (kMode == kMixed) {
-      const float2 r = a.rcp32[g], d = a.r0[g];
-      a.hsd32[k] = make_float4(r.x, r.y, d.x, d.y);
-      if (k < 32 * ps.hps[5]) {
-        const int s = k / kSlice, so = ps.soff[s - ps.hps[0]];
-        if (so >= 0)
-          reinterpret_cast<float4 *>(stage + 16 * so + ps.w[s - ps.hps[0]] * kSlice * 10 + 2 * kSlice * 4)[k % kSlice] =
-              make_float4(r.x, r.y, d.x, d.y);
-      }
-      if (k >= 32 * ps.hps[5]) {
-        // boundary slots: c0 = mean of the averaged neighbours' u0 minus the row's u0 (FP64),
-        // and 1 / (number averaged), for halo_boundary
-        const int s = k / kSlice, lane = k % kSlice;
-        const int w = ps.w[s - ps.hps[0]];
-        const int64_t e0 = ps.e0[s - ps.hps[0]] + lane;
-        double sx = 0.0, sy = 0.0;
-        int n = 0;
-        for (int q = 0; q < w; ++q) {
-          const int jj = a.hcol[e0 + (int64_t)q * kSlice];
-          if (jj == (int)kNoCol) break;
-          const double2 u = a.UV[halo_global(a, ps, jj)];
-          sx = sx + u.x;
-          sy = sy + u.y;
-          ++n;
-        }
-        const double2 u0 = a.UV[g];
-        const double rn = n > 0 ? 1.0 / (double)n : 0.0;
-        a.hsd32[k] = make_float4((float)(sx * rn - u0.x), (float)(sy * rn - u0.y), (float)rn, 0.0f);
-      }
-    } else {
-      a.hrcp[k] = a.rcp[g];
-      a.hrhs[k] = a.rhs[g];
-    }
-  }
-  __syncthreads();
-}
-
-// Halo slots of the working copy from the buffer the neighbours wrote in the last sweep.
-// The patch's halo slots' device rows are kept in shared memory after the working copy
-// (halo_index), which saves one dependent L2 load per sweep.
-template <class T>
-__device__ __forceinline__ void halo_load(const PatchSmem &ps, const int *hidx, T *ld, const T *in) {
-  for (int i = threadIdx.x; i < ps.nh; i += blockDim.x) ld[ps.n_own + i] = in[hidx[i]];
-}
-
-// Own rows of the working copy into a global buffer.
-template <class T>
-__device__ __forceinline__ void halo_store_own(const PatchSmem &ps, const T *ld, T *dst) {
-  for (int i = threadIdx.x; i < ps.n_own; i += blockDim.x) dst[ps.p0 + i] = ld[i];
-}
-
 // Mixed path: u0 += d, d = 0 on every row.
 template <class Team>
 __device__ void phase_fold(const SsaArgs &a, const Team &t) {
@@ -1219,53 +845,6 @@ __device__ __forceinline__ void wait_neighbours(const Args &a, const PatchSmem &
   __syncthreads();
 }
 
-// wait_neighbours and halo_load by the last kFetchWarps warps (the others meanwhile run the
-// rows that read no halo slot); the caller's CTA barrier then orders the halo slots before their
-// readers. The loads of a thread are issued together (up to kFetchBatch in flight).
-template <class T>
-__device__ __forceinline__ void halo_fetch(const SsaArgs &a, const PatchSmem &ps, unsigned int target,
-                                           unsigned int *team_bar, bool wait, const int *hidx, T *ld, const T *in) {
-  const int ft = (int)threadIdx.x - (int)(blockDim.x - kFetchWarps * kSlice);   // 0 .. 127
-  if (wait) {
-    for (int i = ft; i < ps.nsync; i += kFetchWarps * kSlice) {
-      const unsigned int *q = a.prog + 32 * ps.sync[i];
-      unsigned int v = ld_acquire_u32(q);
-      if ((int)(v - target) < 0) {
-        const unsigned long long t0 = globaltimer_ns();
-        unsigned int ns = 16;
-        for (;;) {
-          __nanosleep(ns);
-          if (ns < 64) ns <<= 1;
-          v = ld_acquire_u32(q);
-          if ((int)(v - target) >= 0) break;
-          if (*(volatile unsigned int *)team_bar & kBarrierError) break;   // another CTA failed
-          if ((long long)(globaltimer_ns() - t0) > a.timeout_ns) {
-            atomicCAS(&a.ctl->err, 0, (int)UFE_TIMEOUT);
-            atomicOr(team_bar, kBarrierError);
-            break;
-          }
-        }
-      }
-    }
-    // the fetch warps' barrier (id 1) orders every acquire before their halo loads
-    asm volatile("bar.sync 1, %0;" ::"r"(kFetchWarps * kSlice) : "memory");
-  }
-  constexpr int kStride = kFetchWarps * kSlice;
-  for (int i0 = ft; i0 < ps.nh; i0 += kStride * kFetchBatch) {
-    T v[kFetchBatch];
-#pragma unroll
-    for (int k = 0; k < kFetchBatch; ++k) {
-      const int i = i0 + k * kStride;
-      if (i < ps.nh) v[k] = in[hidx[i]];
-    }
-#pragma unroll
-    for (int k = 0; k < kFetchBatch; ++k) {
-      const int i = i0 + k * kStride;
-      if (i < ps.nh) ld[ps.n_own + i] = v[k];
-    }
-  }
-}
-
 // Lagged decisions (mixed sweeps). After its colour phases each CTA folds its maximum |res|
 // into the ring slot of sweep G (one atomicMax of a key that carries the sweep, kept for the
 // report of the final residual) and, behind a release, adds its arrival to the slot's word:
@@ -1278,9 +857,7 @@ __device__ __forceinline__ void halo_fetch(const SsaArgs &a, const PatchSmem &ps
 // when some are NaN) with a single load. Every CTA reads every sweep of a solve in order (the
 // sweeps left undecided at the end of a linear solve are drained), so that difference holds
 // exactly the sweep's arrivals; a count above the team's size means that the slot was refilled
-// before it was read (cannot happen with lag <= kMaxLag). The halo sweeps' arrival reads the
-// previous sweep's word ahead, its load overlapping the arrival's fence, and the decision uses
-// that value when it already holds the whole sweep.
+// before it was read (cannot happen with lag <= kMaxLag).
 __device__ __forceinline__ unsigned long long lag_increment(unsigned long long mx_bits, double tol, unsigned int G,
                                                             unsigned long long *key) {
   const float r = __double2float_ru(__longlong_as_double((long long)mx_bits));
@@ -1317,29 +894,6 @@ __device__ __forceinline__ void lag_arrive(const SsaArgs &a, unsigned int G, uns
   }
 }
 
-// lag_arrive, then publish_progress(value), under one release: a single fence orders the
-// slot's maximum, and every write of the CTA before the barrier, before both the arrival and
-// the progress counter (a fence followed by relaxed writes is a release of each of them).
-template <class Team>
-__device__ __forceinline__ void lag_arrive_publish(const SsaArgs &a, const Team &t, PatchSmem &ps, unsigned int G,
-                                                   unsigned long long mx_bits, unsigned int value) {
-  // sweep G - 1's word, read ahead for lag_decide: its load overlaps the reduction and the fence
-  unsigned long long pre = 0ull;
-  if (threadIdx.x == 0 && G > 0u)
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(pre) : "l"(&a.ctl->lag_word[(G - 1u) % kLagRing]) : "memory");
-  const unsigned long long x = block_max_u64(mx_bits);
-  if (threadIdx.x == 0) {
-    ps.lag_pre = pre;
-    ps.lag_pre_g = G - 1u;
-    unsigned long long key;
-    const unsigned long long inc = lag_increment(x, a.tol, G, &key);
-    atomicMax(&a.ctl->lag_res[G % kLagRing], key);
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(&a.ctl->lag_word[G % kLagRing]), "l"(inc) : "memory");
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(a.prog + 32 * t.rank()), "r"(value) : "memory");
-  }
-}
-
 // The decision on sweep G for the whole block: 1 converged, 2 diverged, 0 neither, -1 when a
 // bounded wait ran out, the team's error bit is set, or the slot was refilled early.
 template <class Team>
@@ -1349,13 +903,7 @@ __device__ __forceinline__ int lag_decide(const SsaArgs &a, const Team &t, Patch
     const unsigned long long *wp = &a.ctl->lag_word[slot];
     const unsigned long long n = (unsigned long long)t.size();
     const unsigned long long prev = ps.lag_prev[slot];
-    unsigned long long d = 0ull;
-    bool have = false;   // the word read ahead holds the whole sweep
-    if (ps.lag_pre_g == G) {
-      d = ps.lag_pre - prev;
-      have = (d & 0xffffull) == n;
-    }
-    if (!have) d = ld_acquire_u64(wp) - prev;
+    unsigned long long d = ld_acquire_u64(wp) - prev;
     int act = 0;
     if ((d & 0xffffull) < n) {
       const unsigned long long t0 = globaltimer_ns();
@@ -1419,7 +967,6 @@ __device__ __forceinline__ bool lag_drain(const SsaArgs &a, const Team &t, Patch
 template <class Args>
 __device__ __forceinline__ void load_patch(const Args &a, int b, PatchSmem &ps) {
   if (threadIdx.x < 8) ps.lag_prev[threadIdx.x] = 0ull;
-  if (threadIdx.x == 0) ps.lag_pre_g = 0xffffffffu;   // nothing read ahead (lag_decide)
   if (threadIdx.x <= kGroups) ps.ps[threadIdx.x] = a.patch_slice[b * (kGroups + 1) + threadIdx.x];
   if (threadIdx.x == 0) {
     ps.edge0 = a.patch_edge0[b];
@@ -1435,75 +982,23 @@ __device__ __forceinline__ void load_patch(const Args &a, int b, PatchSmem &ps) 
   __syncthreads();
 }
 
-// Patch b's halo program (phase slice ranges and slice table), own rows, halo slots and the
-// patches of its start-of-sweep wait into shared memory.
-__device__ __forceinline__ void load_patch_halo(const SsaArgs &a, int b, PatchSmem &ps) {
-  if (threadIdx.x < 8) ps.lag_prev[threadIdx.x] = 0ull;
-  if (threadIdx.x == 0) ps.lag_pre_g = 0xffffffffu;
-  if (threadIdx.x <= kGroups) ps.ps[threadIdx.x] = a.patch_slice[b * (kGroups + 1) + threadIdx.x];
-  if (threadIdx.x < 8) ps.hps[threadIdx.x] = a.hp_slice[b * 7 + threadIdx.x];
-  if (threadIdx.x == 0) {
-    ps.nsync = a.hsync_ptr[b + 1] - a.hsync_ptr[b];
-    ps.hsplit = a.hp_split[b];
-    ps.hl0 = a.hload_ptr[b];
-    ps.nh = a.hload_ptr[b + 1] - a.hload_ptr[b];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ps.p0 = ps.ps[0] * kSlice;
-    ps.n_own = (ps.ps[kGroups] - ps.ps[0]) * kSlice;
-  }
-  for (int i = threadIdx.x; i < ps.nsync; i += blockDim.x) ps.sync[i] = a.hsync_list[a.hsync_ptr[b] + i];
-  for (int s = ps.hps[0] + threadIdx.x; s < ps.hps[7]; s += blockDim.x) {
-    ps.e0[s - ps.hps[0]] = a.hslice_e0[s];
-    ps.w[s - ps.hps[0]] = a.hslice_w[s];
-  }
-  __syncthreads();
-}
-
 // The whole solve_SSA of one problem, run by the CTAs of a team (each CTA owns one patch).
 // Returns false when a bounded wait failed; the error is recorded in the problem's control
-// block and the team's barrier counter. kHalo: the halo sweeps (one neighbour wait per
-// sweep, the patch's working copy in shared memory, velocities in three buffers by sweep).
-template <int kMode, class Team, bool kHalo = false>
+// block and the team's barrier counter. The phased sweeps; solve_member_halo runs the halo sweeps.
+template <int kMode, class Team>
 __device__ bool solve_member(const SsaArgs &a, Team &t) {
   constexpr bool kM = kMode == kMixed;
-  using T = typename std::conditional<kM, float2, double2>::type;
   SsaCtl *ctl = a.ctl;
-  unsigned int phases = 0;   // colour phases (halo sweeps: sweeps) completed by this patch
+  unsigned int phases = 0;   // colour phases completed by this patch
   const bool leader = t.rank() == 0 && threadIdx.x == 0;
   __shared__ PatchSmem ps;
-  if constexpr (kHalo) load_patch_halo(a, t.rank(), ps);
-  else load_patch(a, t.rank(), ps);
+  load_patch(a, t.rank(), ps);
   extern __shared__ __align__(16) unsigned char ufe_local_rows[];
   const LocalRows lc{ufe_local_rows, ps.ps[0] * kSlice,
                      (kMode != kExact64 && a.local_rows) ? (ps.ps[kGroups] - ps.ps[0]) * kSlice : 0};
-  T *const hbuf0 = reinterpret_cast<T *>(kM ? (void *)a.dUV : (void *)a.UV);
-  T *const hbuf1 = reinterpret_cast<T *>(kM ? (void *)a.dUVb : (void *)a.UVb);
-  T *const hbuf2 = reinterpret_cast<T *>(kM ? (void *)a.dUVc : (void *)a.UVc);
-  T *const hld = reinterpret_cast<T *>(ufe_local_rows);
-  int *const hidx = reinterpret_cast<int *>(ufe_local_rows + (size_t)a.halo_index_off);
-  unsigned char *const hstage = ufe_local_rows + (size_t)a.stage_off;
-  if constexpr (kHalo) {
-    for (int i = threadIdx.x; i < ps.nh; i += blockDim.x) hidx[i] = a.hload_dev[ps.hl0 + i];
-    __syncthreads();
-    if constexpr (kM) halo_stage(a, ps, hstage);
-  }
   // (Re)load the mirror from global memory: at the start and after the grid-wide phases
-  // that rewrite every row (fold, reset). Halo sweeps: the own rows of the working copy, also
-  // copied into the other two buffers, which then hold every row that no sweep writes
-  // (Dirichlet rows) as well.
+  // that rewrite every row (fold, reset).
   auto reload = [&]() {
-    if constexpr (kHalo) {
-      for (int i = threadIdx.x; i < ps.n_own; i += blockDim.x) {
-        const T v = hbuf0[ps.p0 + i];
-        hld[i] = v;
-        hbuf1[ps.p0 + i] = v;
-        hbuf2[ps.p0 + i] = v;
-      }
-      __syncthreads();
-      return;
-    }
     if (!lc.n) return;
     for (int i = threadIdx.x; i < lc.n; i += blockDim.x) {
       if (kM) static_cast<float2 *>(lc.base)[i] = a.dUV[lc.p0 + i];
@@ -1546,150 +1041,6 @@ __device__ bool solve_member(const SsaArgs &a, Team &t) {
     bool lin_done = false;
     int did_reset = 0;
     double maxres = 0.0;
-    if constexpr (kHalo) {
-      // Halo sweeps. Every patch's rows of a sweep go to the next of three buffers (cur: the one
-      // holding the latest rows). A sweep first runs colour 1's own rows that read no halo slot
-      // (their inputs are own rows of the working copy; the buffer it writes was last read by
-      // the neighbouring patches two sweeps ago, before they completed the sweep this patch
-      // waited for at the start of the previous one), then waits once for the patches whose rows
-      // it reads and that read its rows (they finished the previous sweep, so buffer cur holds
-      // their rows), loads its halo slots, and runs the rest of the seven phases on its working
-      // copy with CTA barriers only. Sync points commit the own rows to the canonical buffer.
-      constexpr bool kLag = kM && kMixedLag > 0;
-      auto hb = [&](int i) { return i == 0 ? hbuf0 : i == 1 ? hbuf1 : hbuf2; };
-      int cur = 0;
-      bool synced = true;
-      int decided = 0;
-      const unsigned int base = gsweep;
-      halo_refresh<kMode>(a, ps, hstage);
-      UFE_TM(kTmOther);
-      while (!lin_done && sweeps < a.max_inner) {
-        ++sweeps;
-        UFE_TM_COUNT(kTmSweeps);
-        const unsigned int G = gsweep++;
-        const int slot = sweeps % 3;
-        if (!kLag && leader) ctl->maxres[(sweeps + 1) % 3] = 0ull;
-        T *const out = hb(cur == 2 ? 0 : cur + 1);
-        auto colour = [&](int s_begin, int s_end, int nw) -> unsigned long long {
-          if constexpr (kM) return halo_colour32(a, ps, s_begin, s_end, nw, hstage, hidx, hld, out);
-          else return halo_colour64<kMode == kExact64>(a, ps, s_begin, s_end, nw, hld, out);
-        };
-        // the last kFetchWarps warps wait for the neighbouring patches and load the halo slots
-        // while the others run colour 1's halo-free rows
-        // (the FP64 modes, with a team barrier after every sweep, wait for nothing here and run
-        // colour 1 whole)
-        const int nwarps = blockDim.x >> 5;
-        unsigned long long mx = 0ull;
-        if constexpr (kLag) {
-          if ((int)(threadIdx.x >> 5) < nwarps - kFetchWarps) mx = colour(ps.hps[0], ps.hsplit, nwarps - kFetchWarps);
-          else halo_fetch(a, ps, phases, t.bar(), !synced, hidx, hld, hb(cur));
-        } else {
-          halo_load(ps, hidx, hld, hb(cur));
-        }
-        __syncthreads();
-        UFE_TM(kTmWaitColour);
-        for (int f = 0; f < 5; ++f) {
-          const int s_begin = f == 0 && kLag ? ps.hsplit : ps.hps[f];
-          if (ps.hps[f + 1] == s_begin) continue;
-          const unsigned long long m = colour(s_begin, ps.hps[f + 1], nwarps);
-          mx = m > mx ? m : mx;
-          __syncthreads();
-          UFE_TM_SUB(kTmColour0 + f);
-        }
-        UFE_TM(kTmColour);
-        for (int f = 5; f < 7; ++f) {
-          if (ps.hps[f + 1] == ps.hps[f]) continue;
-          halo_boundary<kM>(a, ps, f, hld, out);
-          __syncthreads();
-        }
-        UFE_TM(kTmBoundary);
-        cur = cur == 2 ? 0 : cur + 1;
-        if constexpr (kLag) {
-          ++phases;
-          lag_arrive_publish(a, t, ps, G, mx, phases);
-          UFE_TM(kTmArrive);
-          synced = false;
-          const bool refold_now = a.refold > 0 && sweeps % a.refold == 0;
-          const bool sync_point = sweeps == a.max_inner || refold_now;
-          if (sync_point) {
-            if (cur) halo_store_own(ps, hld, hbuf0);
-            cur = 0;
-            UFE_GRID_SYNC();
-            synced = true;
-            UFE_TM(kTmGrid);
-          }
-          const int upto = sync_point ? sweeps : sweeps - kMixedLag;
-          int act = 0;             // 1: converged, 2: diverged
-          while (decided < upto && act == 0) {
-            ++decided;
-            act = lag_decide(a, t, ps, base + (unsigned)(decided - 1));
-            if (act < 0) {
-              if (threadIdx.x == 0) a.prog[32 * t.rank()] = 0x7fffffffu;
-              return false;
-            }
-          }
-          UFE_TM(kTmDecide);
-          if (act == 1) {
-            lin_done = true;
-          } else if (act == 2) {
-            if (!synced) { UFE_GRID_SYNC(); synced = true; }
-            phase_zero_velocity(a, t, kM);
-            UFE_GRID_SYNC();
-            reload();
-            cur = 0;
-            did_reset = 1;
-            lin_done = true;
-          } else if (sweeps == a.max_inner) {
-            if (leader) ctl->not_converged += 1;
-          } else if (refold_now) {
-            phase_fold(a, t);
-            UFE_GRID_SYNC();
-            reload();
-            phase_defect(a, t);
-            UFE_GRID_SYNC();
-            halo_refresh<kMode>(a, ps, hstage);
-          }
-          UFE_TM(kTmOther);
-        } else {
-          block_max_to(&ctl->maxres[slot], mx);
-          UFE_TM(kTmArrive);
-          UFE_GRID_SYNC();
-          UFE_TM(kTmGrid);
-          maxres = __longlong_as_double((long long)*(volatile unsigned long long *)&ctl->maxres[slot]);
-          if (maxres < a.tol) {
-            lin_done = true;
-          } else if (maxres > 1e6) {
-            phase_zero_velocity(a, t, kM);
-            UFE_GRID_SYNC();
-            reload();
-            cur = 0;
-            did_reset = 1;
-            lin_done = true;
-          } else if (sweeps == a.max_inner) {
-            if (leader) ctl->not_converged += 1;
-          } else if (kM && a.refold > 0 && sweeps % a.refold == 0) {
-            if (cur) halo_store_own(ps, hld, hbuf0);
-            cur = 0;
-            UFE_GRID_SYNC();
-            phase_fold(a, t);
-            UFE_GRID_SYNC();
-            reload();
-            phase_defect(a, t);
-            UFE_GRID_SYNC();
-            halo_refresh<kMode>(a, ps, hstage);
-          }
-          UFE_TM(kTmOther);
-        }
-      }
-      if constexpr (kLag) {
-        if (!lag_drain(a, t, ps, base, decided, sweeps, leader, maxres)) return false;
-      }
-      // the final own rows into the canonical buffer before the grid-wide phases read it
-      const bool commit = cur || (kLag && !synced);
-      if (cur) halo_store_own(ps, hld, hbuf0);
-      if (commit) UFE_GRID_SYNC();
-      UFE_TM(kTmGrid);
-    } else
     if constexpr (kM && kMixedLag > 0) {
       // Mixed sweeps with lagged decisions: the boundary phase is a counted phase and the next
       // sweep's first colour waits for the neighbours' boundary rows, so no team barrier
@@ -1846,6 +1197,10 @@ __device__ bool solve_member(const SsaArgs &a, Team &t) {
 #undef UFE_GRID_SYNC
 }
 
+}  // namespace ufe
+#include "ufe_halo.cuh"
+namespace ufe {
+
 // Stage the argument block in shared memory (it is read on every phase by every thread).
 __device__ __forceinline__ void stage_args(SsaArgs &dst, const SsaArgs *src) {
   const int n = (int)(sizeof(SsaArgs) / sizeof(int));
@@ -1858,9 +1213,11 @@ __device__ __forceinline__ void stage_args(SsaArgs &dst, const SsaArgs *src) {
 // Single solve: the whole grid is one team; the argument block stays in the kernel's
 // parameter space (constant bank operands cost no registers).
 template <int kMode, bool kHalo>
-__global__ void __launch_bounds__(kHalo ? kHaloBlock : kSsaBlock, kCtasPerSm) ssa_persistent(const SsaArgs a) {
+__global__ void __launch_bounds__(kHalo ? kHaloBlock : kSsaBlock, kCtasPerSm)
+    ssa_persistent(const __grid_constant__ SsaArgs a) {
   GridTeam t{&a.ctl->bar_count, 0u};
-  solve_member<kMode, GridTeam, kHalo>(a, t);
+  if constexpr (kHalo) solve_member_halo<kMode>(a, t);
+  else solve_member<kMode>(a, t);
 }
 
 // Ensemble of independent solves in one launch. The grid is cut into teams; a team of T
@@ -1900,7 +1257,10 @@ __global__ void __launch_bounds__(kBlock, kPerSm) ssa_batched(const BatchArgs b)
     const unsigned int m = *(volatile unsigned int *)&b.team_member[32 * team];
     if (m >= (unsigned)b.n_members) return;
     stage_args(a, b.members + m);
-    if (!solve_member<kMode, SubTeam, kHalo>(a, t)) {
+    bool ok;
+    if constexpr (kHalo) ok = solve_member_halo<kMode>(a, t);
+    else ok = solve_member<kMode>(a, t);
+    if (!ok) {
       if (threadIdx.x == 0) atomicCAS(b.err, 0, (int)UFE_TIMEOUT);
       return;
     }
@@ -2520,10 +1880,8 @@ struct SsaWork {
   double *f = nullptr;           // Hi, Hb, SL, hx, hy, Af, beta, tau, phi, eta, Na, Nb, S
   double2 *UV = nullptr, *rhs = nullptr, *euv = nullptr, *rcp = nullptr;
   float2 *dUV = nullptr, *r0 = nullptr, *rcp32 = nullptr;
-  double2 *UVb = nullptr, *UVc = nullptr;   // halo sweeps: second and third velocity buffers (FP64 modes)
-  float2 *dUVb = nullptr, *dUVc = nullptr;  // halo sweeps: second and third correction buffers (mixed)
-  float4 *hsd32 = nullptr;       // halo sweeps: per-slot row data (mixed)
-  double2 *hrcp = nullptr, *hrhs = nullptr;   // halo sweeps: per-slot row data (fast FP64)
+  double2 *hundo = nullptr;              // halo sweeps, FP64: values before the last update, per program slot
+  unsigned long long *hxch = nullptr;    // halo sweeps: exchange buffers
   float4 *bc0 = nullptr;         // mixed: boundary offsets per edge ordinal
   uint8_t *skip = nullptr;
   double *rn_part = nullptr;
@@ -2546,7 +1904,7 @@ void ssa_free(SsaWork *w) {
   if (!w) return;
   void *ptrs[] = {w->stage_in, w->stage_out, w->gl_int, w->gl_dbl, w->f, w->UV, w->rhs, w->euv,
                   w->rcp, w->dUV, w->r0, w->rcp32, w->skip, w->rn_part, w->prog, w->ctl, w->fh,
-                  w->UVb, w->dUVb, w->UVc, w->dUVc, w->hsd32, w->hrcp, w->hrhs, w->bc0};
+                  w->hundo, w->hxch, w->bc0};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (w->ctl_host) cudaFreeHost(w->ctl_host);
@@ -2560,6 +1918,10 @@ namespace {
 enum { F_HI, F_HB, F_SL, F_HX, F_HY, F_AF, F_BETA, F_TAU, F_PHI, F_ETA, F_NA, F_NB, F_S, F_COUNT };
 // stage_in layout (doubles): Aa block 6*nV, Ac block 6*nAc, beta nA, U nV, V nV, Ux nAc, Uy nAc, N nA
 // stage_out layout: U nV, V nV, Ux nAc, Uy nAc, Up nAc, Uo nAc, N nA, eta nA, S nA, tau nA, phi nA
+
+// The exchange buffers of the halo sweeps: two words per exported row (mixed), four (FP64).
+size_t exchange_stride(const DevMesh &m, int mode) { return (size_t)m.n_export * (mode == kMixed ? 2 : 4); }
+size_t exchange_bytes(const DevMesh &m, int mode) { return kXchBufs * exchange_stride(m, mode) * sizeof(unsigned long long); }
 
 int ensure_work(ufe_mesh_h h) {
   if (h->ssa) return UFE_OK;
@@ -2582,28 +1944,23 @@ int ensure_work(ufe_mesh_h h) {
   if (!rc) rc = cuda_status(cudaMalloc(&w->rcp32, (size_t)m.nP * sizeof(float2)), "ssa rcp32");
   if (!rc) rc = cuda_status(cudaMalloc(&w->skip, (size_t)m.nP), "ssa skip");
   if (!rc) rc = cuda_status(cudaMalloc(&w->bc0, ((size_t)m.n_edge_total + 1) * sizeof(float4)), "ssa bc0");
-  if (!rc && m.has_halo) rc = cuda_status(cudaMalloc(&w->UVb, (size_t)m.nP * sizeof(double2)), "ssa UVb");
-  if (!rc && m.has_halo) rc = cuda_status(cudaMalloc(&w->dUVb, (size_t)m.nP * sizeof(float2)), "ssa dUVb");
-  if (!rc && m.has_halo) rc = cuda_status(cudaMalloc(&w->UVc, (size_t)m.nP * sizeof(double2)), "ssa UVc");
-  if (!rc && m.has_halo) rc = cuda_status(cudaMalloc(&w->dUVc, (size_t)m.nP * sizeof(float2)), "ssa dUVc");
-  const size_t nslots = (size_t)m.n_hslices * kSlice;
-  if (!rc && m.has_halo) rc = cuda_status(cudaMalloc(&w->hsd32, nslots * sizeof(float4)), "ssa hsd32");
-  if (!rc && m.has_halo) rc = cuda_status(cudaMalloc(&w->hrcp, nslots * sizeof(double2)), "ssa hrcp");
-  if (!rc && m.has_halo) rc = cuda_status(cudaMalloc(&w->hrhs, nslots * sizeof(double2)), "ssa hrhs");
+  if (!rc && m.has_halo) rc = cuda_status(cudaMalloc(&w->hundo, (size_t)m.n_hslices * kSlice * sizeof(double2)), "ssa undo");
+  if (!rc && m.has_halo) rc = cuda_status(cudaMalloc(&w->hxch, exchange_bytes(m, kFast64) + 16), "ssa exchange");
   if (!rc) rc = cuda_status(cudaMalloc(&w->ctl, sizeof(SsaCtl)), "ssa ctl");
   if (!rc) rc = cuda_status(cudaMallocHost(&w->ctl_host, sizeof(SsaCtl)), "ssa ctl host");
   if (!rc) rc = cuda_status(cudaEventCreate(&w->ev0), "event");
   if (!rc) rc = cuda_status(cudaEventCreate(&w->ev1), "event");
   if (!rc) rc = cuda_status(cudaMemsetAsync(w->skip, 0, (size_t)m.nP, h->stream), "memset skip");
   // Persistent grid: every CTA co-resident (cooperative launch), one CTA of 1024 threads per SM.
-  const void *kernels[5] = {(const void *)ssa_persistent<kExact64, false>, (const void *)ssa_persistent<kFast64, false>,
-                            (const void *)ssa_persistent<kMixed, false>, (const void *)ssa_persistent<kFast64, true>,
-                            (const void *)ssa_persistent<kMixed, true>};
+  const void *kernels[6] = {(const void *)ssa_persistent<kExact64, false>, (const void *)ssa_persistent<kFast64, false>,
+                            (const void *)ssa_persistent<kMixed, false>, (const void *)ssa_persistent<kExact64, true>,
+                            (const void *)ssa_persistent<kFast64, true>, (const void *)ssa_persistent<kMixed, true>};
   int gmax = 0;
-  for (int k = 0; k < 5 && !rc; ++k) {
+  for (int k = 0; k < 6 && !rc; ++k) {
     if (k >= 3 && !m.has_halo) break;
     int per_sm = 0;
-    rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[k], k >= 3 ? kHaloBlock : w->block, 0),
+    rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[k],
+                                                                   k >= 3 ? kHaloBlock : w->block, 0),
                      "occupancy");
     if (!rc && per_sm * h->num_sms < m.n_patch) {
       set_error("ssa kernel: not enough co-resident CTAs for one per patch");
@@ -2612,7 +1969,7 @@ int ensure_work(ufe_mesh_h h) {
     if (k < 3) w->grid[k] = m.n_patch;   // one CTA per patch (n_patch <= kCtasPerSm * number of SMs)
     gmax = gmax > m.n_patch ? gmax : m.n_patch;
   }
-  if (!rc) rc = cuda_status(cudaMalloc(&w->rn_part, 2 * (size_t)gmax * sizeof(double)), "rn_part");
+  if (!rc) rc = cuda_status(cudaMalloc(&w->rn_part, (2 + kLagRing) * (size_t)gmax * sizeof(double)), "rn_part");
   if (!rc) rc = cuda_status(cudaMalloc(&w->prog, 32 * (size_t)gmax * sizeof(unsigned int)), "progress counters");
   if (rc) { ssa_free(w); return rc; }
   h->ssa = w;
@@ -2786,12 +2143,6 @@ int launch_prepare(ufe_mesh_h h, const ufe_params *p, cudaStream_t s, SsaArgs *a
   a->s3Nxy = m.s3Nxy; a->h_nxy32 = m.h_nxy32; a->s3Nxy32 = m.s3Nxy32; a->bnd_ptr = m.bnd_ptr; a->bnd_nbr = m.bnd_nbr;
   a->slice_e0 = m.slice_e0; a->slice_w = m.slice_w; a->slice_g = m.slice_g; a->patch_slice = m.patch_slice;
   a->patch_edge0 = m.patch_edge0; a->edge_row = m.edge_row; a->sync_ptr = m.sync_ptr; a->sync_list = m.sync_list;
-  a->hp_slice = m.hp_slice; a->hslice_e0 = m.hslice_e0; a->hslice_w = m.hslice_w; a->hrow_l = m.hrow_l;
-  a->hrow_g = m.hrow_g; a->hcol = m.hcol; a->hcuv32 = m.hcuv32; a->hcuv = m.hcuv; a->hload_ptr = m.hload_ptr;
-  a->hload_dev = m.hload_dev; a->hsync_ptr = m.hsync_ptr; a->hsync_list = m.hsync_list;
-  a->UVb = w->UVb; a->dUVb = w->dUVb; a->UVc = w->UVc; a->dUVc = w->dUVc; a->hs3_32 = m.hs3_32; a->hs3 = m.hs3;
-  a->hp_split = m.hp_split;
-  a->hsd32 = w->hsd32; a->hrcp = w->hrcp; a->hrhs = w->hrhs;
   a->bc0 = w->bc0; a->n_edge = m.n_edge_total;
   a->prog = w->prog; a->nP = m.nP; a->nSlices = m.nSlices; a->ncm = m.ncm;
   a->Hi = fl.Hi; a->Hb = fl.Hb; a->SL = fl.SL; a->hx = fl.hx; a->hy = fl.hy; a->Af = fl.Af;
@@ -2815,6 +2166,25 @@ int launch_prepare(ufe_mesh_h h, const ufe_params *p, cudaStream_t s, SsaArgs *a
   a->fp32_visc = p->mixed_fp32_viscosity != 0;
   a->timeout_ns = wait_timeout_ns();
   return rc;
+}
+
+// The halo sweeps' part of the argument block; clears the exchange buffers (their tags).
+int prepare_halo(ufe_mesh_h h, int mode, cudaStream_t s, SsaArgs *a) {
+  SsaWork *w = h->ssa;
+  const DevMesh &m = h->m;
+  a->hp_slice = m.hp_slice; a->hp_split = m.hp_split; a->hslice_w = m.hslice_w; a->hrow_g = m.hrow_g;
+  a->hslice_b0 = mode == kMixed ? m.hslice_b32 : m.hslice_b64;
+  a->hprog = mode == kMixed ? m.hprog32 : m.hprog64;
+  a->hload_ptr = m.hload_ptr; a->hload_dev = m.hload_dev; a->hload_ex = m.hload_ex; a->hex_ptr = m.hex_ptr;
+  a->hundo = w->hundo; a->hxch = w->hxch;
+  a->xch_stride = exchange_stride(m, mode);
+  a->res_part = w->rn_part + 2 * (size_t)m.n_patch;
+  float t = (float)a->tol;
+  if ((double)t < a->tol) t = std::nextafterf(t, INFINITY);
+  a->tol32 = t;
+  a->omega32 = (float)a->omega;
+  if (m.n_export == 0) return UFE_OK;
+  return cuda_status(cudaMemsetAsync(w->hxch, 0, exchange_bytes(m, mode), s), "memset exchange");
 }
 
 // Scatter the results back to the caller's order and fetch the control block.
@@ -2869,7 +2239,9 @@ int stats_of(const SsaCtl &c, ufe_ssa_stats *stats, double ms) {
 }
 
 const void *persistent_kernel(int mode, bool halo) {
-  if (halo) return mode == kMixed ? (const void *)ssa_persistent<kMixed, true> : (const void *)ssa_persistent<kFast64, true>;
+  if (halo) return mode == kMixed ? (const void *)ssa_persistent<kMixed, true>
+                   : mode == kFast64 ? (const void *)ssa_persistent<kFast64, true>
+                                     : (const void *)ssa_persistent<kExact64, true>;
   return mode == kMixed ? (const void *)ssa_persistent<kMixed, false>
          : mode == kFast64 ? (const void *)ssa_persistent<kFast64, false>
                            : (const void *)ssa_persistent<kExact64, false>;
@@ -2901,16 +2273,15 @@ extern "C" int ufe_ssa_run(ufe_mesh_h h, const ufe_params *p, ufe_ssa_stats *sta
     // Halo sweeps when the mesh has the program and the largest working copy fits
     // (UFE_SSA_HALO=0 turns them off); else the phased sweeps with the optional mirror.
     const char *henv = std::getenv("UFE_SSA_HALO");
-    // The parity (exact) mode keeps the phased sweeps: without fused multiply-adds it is bound
-    // by the FP64 pipe, and the halo rows' extra updates measured slower there (133 against
-    // 125 us per sweep on the 200k dome).
-    const bool halo = m.has_halo && mode != kExact64 && (size_t)m.max_local * elem <= kLocalRowsMaxBytes &&
+    const bool halo = m.has_halo && ((size_t)m.max_local + 1) * elem <= kLocalRowsMaxBytes &&
                       !(henv && henv[0] == '0');
-    size_t bytes = halo ? (size_t)m.max_local * elem : (size_t)m.max_patch_slices * kSlice * elem;
+    size_t bytes = halo ? ((size_t)m.max_local + 1) * elem : (size_t)m.max_patch_slices * kSlice * elem;
     a.halo_index_off = (int)bytes;
     if (halo) bytes += (size_t)m.max_halo * sizeof(int);
     a.stage_off = (int)((bytes + 15) / 16 * 16);
     a.stage_bytes = 0;
+    if (halo) rc = prepare_halo(h, mode, s, &a);
+    const int block = halo ? kHaloBlock : w->block;
     const char *env = std::getenv("UFE_SSA_LOCAL_ROWS");
     bool local = halo || (mode == kMixed && bytes <= kLocalRowsMaxBytes && !(env && env[0] == '0'));
     const void *fn = persistent_kernel(mode, halo);
@@ -2920,9 +2291,9 @@ extern "C" int ufe_ssa_run(ufe_mesh_h h, const ufe_params *p, ufe_ssa_stats *sta
       // the plain loads if one CTA per SM would then no longer fit.
       cudaFuncAttributes fa;
       int smem_sm = 0, per_sm = 0;
-      rc = cuda_status(cudaFuncGetAttributes(&fa, fn), "function attributes");
+      if (!rc) rc = cuda_status(cudaFuncGetAttributes(&fa, fn), "function attributes");
       if (!rc) rc = cuda_status(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device), "smem per SM");
-      if (!rc && halo && mode == kMixed) {
+      if (!rc && halo) {
         // the resident program slices take what one CTA per SM leaves of the shared memory
         int optin = 0;
         rc = cuda_status(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "smem opt-in");
@@ -2933,7 +2304,7 @@ extern "C" int ufe_ssa_run(ufe_mesh_h h, const ufe_params *p, ufe_ssa_stats *sta
       if (!rc) rc = cuda_status(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attribute");
       const int pct = smem_sm > 0 ? (int)std::min<size_t>(100, (100 * (bytes + fa.sharedSizeBytes + 2048) + smem_sm - 1) / smem_sm) : 100;
       if (!rc) rc = cuda_status(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct), "carveout");
-      if (!rc) rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, halo ? kHaloBlock : w->block, bytes), "occupancy");
+      if (!rc) rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, bytes), "occupancy");
       if (!rc && per_sm * h->num_sms < w->grid[mode]) {
         if (halo) { set_error("ufe_ssa_run: the halo sweeps' working copy leaves no room for one CTA per SM"); rc = UFE_CUDA_ERROR; }
         local = false;
@@ -2943,7 +2314,7 @@ extern "C" int ufe_ssa_run(ufe_mesh_h h, const ufe_params *p, ufe_ssa_stats *sta
     const size_t smem = local ? bytes : 0;
     void *args[] = {(void *)&a};
     if (!rc)
-      rc = cuda_status(cudaLaunchCooperativeKernel(fn, dim3(w->grid[mode]), dim3(halo ? kHaloBlock : w->block), args, smem, s),
+      rc = cuda_status(cudaLaunchCooperativeKernel(fn, dim3(w->grid[mode]), dim3(block), args, smem, s),
                        "ssa_persistent");
   }
   if (!rc) rc = launch_finish(h, s);
@@ -3201,13 +2572,13 @@ void batch_free(ufe_batch_s *b) {
 }
 
 // The batched kernel for a sweep mode and CTA shape (nullptr: not built); halo: the mixed
-// members' halo sweeps.
+// members' halo sweeps, which run half the threads with twice the registers (see kHaloBlock).
 const void *batched_kernel(int mode, int block, bool halo = false) {
   if (halo) {
     switch (mode * 10000 + block) {
-      case kMixed * 10000 + 1024: return (const void *)ssa_batched<kMixed, 1024, 1, true>;
-      case kMixed * 10000 + 512: return (const void *)ssa_batched<kMixed, 512, 2, true>;
-      case kMixed * 10000 + 256: return (const void *)ssa_batched<kMixed, 256, 4, true>;
+      case kMixed * 10000 + 1024: return (const void *)ssa_batched<kMixed, 512, 1, true>;
+      case kMixed * 10000 + 512: return (const void *)ssa_batched<kMixed, 256, 2, true>;
+      case kMixed * 10000 + 256: return (const void *)ssa_batched<kMixed, 128, 4, true>;
       default: return nullptr;
     }
   }
@@ -3299,6 +2670,7 @@ int batch_enqueue(ufe_batch_s *b, const ufe_params *p, int mode) {
       a.halo_index_off = b->halo_index_off;
       a.stage_off = b->halo_stage_off;
       a.stage_bytes = 0;
+      rc = prepare_halo(b->members[m], mode, s, &a);
     }
     if (!rc && solve) {
       const int c = (int)(std::find(pl.class_team_ctas, pl.class_team_ctas + nc, b->team_of_member[m]) -
@@ -3343,7 +2715,7 @@ int batch_enqueue(ufe_batch_s *b, const ufe_params *p, int mode) {
     if (!rc) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)pl.grid_ctas);
-      cfg.blockDim = dim3((unsigned)b->block);
+      cfg.blockDim = dim3((unsigned)(halo ? b->block / 2 : b->block));
       cfg.dynamicSmemBytes = halo ? b->halo_smem : 0;
       cfg.stream = s;
       cudaLaunchAttribute attr[1];
@@ -3437,11 +2809,11 @@ extern "C" int ufe_batch_create(const ufe_mesh_desc *descs, int32_t n, const ufe
     }
     const void *fn = batched_kernel(kMixed, block, true);
     if (all && fn) {
-      const size_t idx_off = (size_t)max_local * sizeof(float2);
+      const size_t idx_off = ((size_t)max_local + 1) * sizeof(float2);
       const size_t stage_off = (idx_off + (size_t)max_halo * sizeof(int) + 15) / 16 * 16;
       int per_sm = 0;
       if (raise_dynamic_smem(fn, b->device, stage_off) &&
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, stage_off) == cudaSuccess &&
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block / 2, stage_off) == cudaSuccess &&
           per_sm * b->num_sms >= b->plan.grid_ctas) {
         b->halo_ok = true;
         b->halo_index_off = (int)idx_off;
