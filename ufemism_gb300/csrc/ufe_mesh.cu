@@ -228,10 +228,14 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
   std::vector<int> order(nA);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key[a] < key[b]; });
-  // Default: one patch per CTA of the single-solve grid, at least kSsaBlock / 2 rows each. A
-  // batched solve asks for its team size instead.
+  // Default: one patch per CTA of the single-solve grid, at least kMinPatchRows rows each. A
+  // batched solve asks for its team size instead. Fewer rows a patch leave each phase fewer slices
+  // per SM, which the FP64 pipe feels at once; below 128 nothing is gained. Per sweep at 512, 256,
+  // 128 and 64 rows: 4k vertices mixed 3.83, 3.48, 3.38, 3.43 us, fast FP64 9.34, 7.87, 7.27, 7.37,
+  // exact 18.5, 13.8, 12.2, 12.2; 740 vertices mixed 3.89, 3.53, 3.48, 3.49, exact 20.6, 14.7, 13.8, 13.6.
+  constexpr int kMinPatchRows = 128, kCoarsePatchRows = 512;
   const int n_patch = n_patch_request > 0 ? std::min(n_patch_request, std::max(1, nA / kSlice))
-                                          : std::max(1, std::min(kCtasPerSm * num_sms, nA / (kSsaBlock / 2)));
+                                          : std::max(1, std::min(kCtasPerSm * num_sms, nA / kMinPatchRows));
   std::vector<int> patch_of(nA);
   std::vector<std::vector<std::vector<int>>> plist(n_patch, std::vector<std::vector<int>>(kGroups));
   for (int k = 0; k < nA; ++k) {
@@ -393,6 +397,8 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
     sync_ptr.push_back((int)sync_list.size());
   }
   m.max_sync = max_sync;
+  if (max_sync > kMaxSync && n_patch_request <= 0 && n_patch > nA / kCoarsePatchRows)   // a coarser cut may do
+    return mesh_create(d, std::max(1, std::min(kCtasPerSm * num_sms, nA / kCoarsePatchRows)), out);
   if (max_sync > kMaxSync) { set_error("ufe_mesh_create: a patch touches too many other patches"); return UFE_BAD_MESH; }
 
   // ---- halo sweep program -----------------------------------------------------------------
