@@ -9,6 +9,7 @@ through the C-ABI; nothing here computes a solve on the CPU.
 from __future__ import annotations
 
 import ctypes as ct
+import threading
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -17,6 +18,78 @@ from . import _native as nat
 
 ZETA_DEFAULT = np.array([0.00, 0.10, 0.20, 0.30, 0.40, 0.50, 0.60, 0.70, 0.80, 0.90,
                          0.925, 0.95, 0.975, 0.99, 1.00])  # configuration_module.f90:124-126
+
+
+class _HostPool:
+    """Host memory of results that have been dropped, for the next results.
+
+    A fresh result array costs its page faults (about 50 us per MB on the GB300's host, against
+    6 us per MB for the copy from the device), so blocks of a page or more are handed out again
+    once no array or view uses them. A block belongs to the array it backs until that array, and
+    every view of it, is gone (the lease is the array's buffer). At most ``limit`` idle bytes are
+    kept; blocks beyond that, and all idle ones on ``release`` (when a mesh or a batch is closed),
+    go back to the allocator. Safe with several threads.
+    """
+
+    def __init__(self, limit: int = 512 << 20, smallest: int = 64 << 10):
+        self.limit, self.smallest = limit, smallest
+        self._idle: dict = {}
+        self._bytes = 0
+        self._lock = threading.RLock()   # a lease may end (in a collection) while its thread holds the lock
+
+    def array(self, shape, dtype=np.float64, order: str = "C"):
+        """An uninitialised array."""
+        shape = (shape,) if np.isscalar(shape) else tuple(shape)
+        dtype = np.dtype(dtype)
+        nbytes = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
+        if nbytes < self.smallest:
+            return np.empty(shape, dtype, order=order)
+        size = -(-nbytes // self.smallest) * self.smallest
+        with self._lock:
+            blocks = self._idle.get(size)
+            block = blocks.pop() if blocks else None
+            if block is not None:
+                self._bytes -= size
+        if block is None:
+            block = np.empty(size, np.uint8)
+        return np.frombuffer(_Lease(self, block), dtype, nbytes // dtype.itemsize).reshape(shape, order=order)
+
+    def zeros(self, shape, dtype=np.float64, order: str = "C"):
+        a = self.array(shape, dtype, order)
+        a.fill(0)
+        return a
+
+    def give_back(self, block):
+        with self._lock:
+            if self._bytes + block.size <= self.limit:
+                self._idle.setdefault(block.size, []).append(block)
+                self._bytes += block.size
+
+    def release(self):
+        with self._lock:
+            self._idle.clear()
+            self._bytes = 0
+
+
+class _Lease:
+    """One array's use of a pool block (the buffer that the array is made from)."""
+
+    def __init__(self, pool, block):
+        self._pool, self._block = pool, block
+
+    def __buffer__(self, flags):
+        return memoryview(self._block)
+
+    def __del__(self):
+        self._pool.give_back(self._block)
+
+
+_pool = _HostPool()
+
+
+def release_host_memory() -> None:
+    """Return the idle memory kept for result arrays to the allocator."""
+    _pool.release()
 
 
 def default_params(**kw) -> dict:
@@ -167,17 +240,23 @@ def _ssa_structs(nV, nAc, nA, fields: dict, warm: dict | None):
     si, keep = _ssa_in(fields)
     warm = warm or {}
     io = {}
-    for k, n in (("U_SSA", nV), ("V_SSA", nV), ("Ux_SSA_Ac", nAc), ("Uy_SSA_Ac", nAc)):
-        io[k] = np.array(warm.get(k, np.zeros(n)), dtype=np.float64, copy=True)
-    io["N_AaAc"] = np.array(warm.get("N_AaAc", np.zeros(nA)), dtype=np.float64, copy=True)
+    for k, n in (("U_SSA", nV), ("V_SSA", nV), ("Ux_SSA_Ac", nAc), ("Uy_SSA_Ac", nAc), ("N_AaAc", nA)):
+        if k not in warm:
+            io[k] = _pool.zeros(n)
+        elif np.shape(warm[k]) == (n,):
+            io[k] = _pool.array(n)
+            io[k][:] = warm[k]
+        else:
+            io[k] = np.array(warm[k], dtype=np.float64, copy=True)
     sio = nat.SsaInout(*(io[k].ctypes.data for k in ("U_SSA", "V_SSA", "Ux_SSA_Ac", "Uy_SSA_Ac", "N_AaAc")))
     return si, sio, io, keep
 
 
 def _download_structs(nV, nAc, nA):
-    io = {k: np.zeros(nV) for k in ("U_SSA", "V_SSA")}
-    io.update({k: np.zeros(nAc) for k in ("Ux_SSA_Ac", "Uy_SSA_Ac", "Up_SSA_Ac", "Uo_SSA_Ac")})
-    io.update({k: np.zeros(nA) for k in ("N_AaAc", "eta_AaAc", "S_AaAc", "tau_c_AaAc", "phi_fric_AaAc")})
+    io = {k: _pool.array(nV) for k in ("U_SSA", "V_SSA")}
+    io.update({k: _pool.array(nAc) for k in ("Ux_SSA_Ac", "Uy_SSA_Ac", "Up_SSA_Ac", "Uo_SSA_Ac")})
+    # zero: not written after the early-out of a solve without grounded ice
+    io.update({k: _pool.zeros(nA) for k in ("N_AaAc", "eta_AaAc", "S_AaAc", "tau_c_AaAc", "phi_fric_AaAc")})
     sio = nat.SsaInout(*(io[k].ctypes.data for k in ("U_SSA", "V_SSA", "Ux_SSA_Ac", "Uy_SSA_Ac", "N_AaAc")))
     so = nat.SsaOut(*(io[k].ctypes.data for k in ("Up_SSA_Ac", "Uo_SSA_Ac", "eta_AaAc", "S_AaAc", "tau_c_AaAc",
                                                    "phi_fric_AaAc")))
@@ -210,6 +289,7 @@ class DeviceMesh:
         if getattr(self, "_h", None):
             nat.load().ufe_mesh_destroy(self._h)
             self._h = None
+            _pool.release()   # the idle blocks have this mesh's sizes
 
     def __del__(self):
         try:
@@ -235,8 +315,8 @@ class DeviceMesh:
         L = nat.load()
         if buffers is None:
             si, sio, io, keep = self._ssa_structs(fields, warm)
-            out = {k: np.zeros(self.nAc) for k in ("Up_SSA_Ac", "Uo_SSA_Ac")}
-            out.update({k: np.zeros(self.nVAaAc) for k in ("eta_AaAc", "S_AaAc", "tau_c_AaAc", "phi_fric_AaAc")})
+            out = {k: _pool.array(self.nAc) for k in ("Up_SSA_Ac", "Uo_SSA_Ac")}
+            out.update({k: _pool.array(self.nVAaAc) for k in ("eta_AaAc", "S_AaAc", "tau_c_AaAc", "phi_fric_AaAc")})
         else:
             if warm is not None:
                 raise ValueError("with buffers the warm start is the buffers' content")
@@ -251,6 +331,15 @@ class DeviceMesh:
         rc = L.ufe_ssa_solve(self._h, ct.byref(ps), ct.byref(si), ct.byref(sio), ct.byref(so), ct.byref(st))
         if check and rc < 0:
             raise nat.UfeError(rc, "ufe_ssa_solve")
+        if buffers is None:   # what this call did not write is zero
+            if rc < 0 and rc != nat.UFE_DIVERGED:
+                unwritten = tuple(out)
+            elif st.picard_iterations == 0:   # the early-out: no grounded ice, or zero_velocities
+                unwritten = ("eta_AaAc", "S_AaAc", "tau_c_AaAc", "phi_fric_AaAc")
+            else:
+                unwritten = ()
+            for k in unwritten:
+                out[k].fill(0)
         out.update(io)
         return rc, out, stats_dict(st)
 
@@ -289,7 +378,7 @@ class DeviceMesh:
         L = nat.load()
         keep = [np.ascontiguousarray(dJ[k], dtype=np.float64) for k in ("U_SSA", "V_SSA", "Ux_SSA_Ac", "Uy_SSA_Ac")]
         vin = nat.VjpIn(*(a.ctypes.data for a in keep))
-        out = {k: np.zeros(self.nVAaAc) for k in nat.VJP_OUT_FIELDS if k != "dJ_dHi"}
+        out = {k: _pool.zeros(self.nVAaAc) for k in nat.VJP_OUT_FIELDS if k != "dJ_dHi"}
         geom = None
         if geom_mesh is not None:
             gm = geom_mesh
@@ -301,7 +390,7 @@ class DeviceMesh:
                       Nx_Ac=_f64(gm.Nx_Ac), Ny_Ac=_f64(gm.Ny_Ac))
             keep.append(gk)
             geom = nat.VjpGeom(*(_ptr(gk[k]) for k in ("nC", "C", "Nx", "Ny", "Aci", "Nx_Ac", "Ny_Ac")))
-            out["dJ_dHi"] = np.zeros(self.nV)
+            out["dJ_dHi"] = _pool.zeros(self.nV)
         vo = nat.VjpOut(*(_ptr(out.get(k)) for k in nat.VJP_OUT_FIELDS))
         vp = nat.VjpParams(tol, max_sweeps, omega, method, restart, sweeps_per_iteration)
         ps, _z = _params_struct(params)
@@ -317,7 +406,7 @@ class DeviceMesh:
         """bottom_frictional_heating from the last solve (ufe_ssa_frictional_heating)."""
         L = nat.load()
         m = np.ascontiguousarray(mask_sheet, dtype=np.int32)
-        out = np.zeros(self.nV)
+        out = _pool.array(self.nV)
         rc = L.ufe_ssa_frictional_heating(self._h, m.ctypes.data, out.ctypes.data)
         if rc != nat.UFE_OK:
             raise nat.UfeError(rc, "ufe_ssa_frictional_heating")
@@ -344,7 +433,7 @@ class DeviceMesh:
         out = {}
         for k in nat.GEOM_OUT_FIELDS:
             n = self.nAc if k.endswith("_Ac") else self.nV
-            out[k] = np.zeros(n, dtype=np.int32 if k in ints else np.float64)
+            out[k] = _pool.array(n, dtype=np.int32 if k in ints else np.float64)
         go = nat.GeometryOut(*(out[k].ctypes.data for k in nat.GEOM_OUT_FIELDS))
         arrs = [np.ascontiguousarray(a, dtype=np.float64) for a in (Hi, Hb, SL)]
         rc = L.ufe_geometry_update(self._h, *(a.ctypes.data for a in arrs), ct.byref(go))
@@ -357,7 +446,7 @@ class DeviceMesh:
         mask_<name> (nV) and mask_<name>_Ac (nAc) for each of nat.MASK_NAMES, plus the type
         masks mask (nV) and mask_Ac (nAc)."""
         L = nat.load()
-        out = {k: np.zeros(self.nAc if k.endswith("_Ac") else self.nV, dtype=np.int32) for k in nat.MASK_OUT_FIELDS}
+        out = {k: _pool.array(self.nAc if k.endswith("_Ac") else self.nV, dtype=np.int32) for k in nat.MASK_OUT_FIELDS}
         mo = nat.MaskOut(*(out[k].ctypes.data for k in nat.MASK_OUT_FIELDS))
         rc = L.ufe_geometry_masks(self._h, ct.byref(mo))
         if rc != nat.UFE_OK:
@@ -385,11 +474,11 @@ class DeviceMesh:
         L = nat.load()
         nZ = len(params["zeta"])
         A = None if A_flow_Ac is None else np.asfortranarray(A_flow_Ac, dtype=np.float64)
-        out = dict(D_SIA_3D_Ac=np.zeros((self.nAc, nZ), order="F"))
+        out = dict(D_SIA_3D_Ac=_pool.array((self.nAc, nZ), order="F"))
         for k in ("D_SIA_Ac", "Ux_SIA_Ac", "Uy_SIA_Ac", "Up_SIA_Ac", "Uo_SIA_Ac"):
-            out[k] = np.zeros(self.nAc)
+            out[k] = _pool.array(self.nAc)
         for k in ("U_SIA", "V_SIA", "D_SIA"):
-            out[k] = np.zeros(self.nV)
+            out[k] = _pool.array(self.nV)
         so = nat.SiaOut(*(_ptr(out[k]) for k in ("D_SIA_3D_Ac", "D_SIA_Ac", "Ux_SIA_Ac", "Uy_SIA_Ac", "Up_SIA_Ac",
                                                   "Uo_SIA_Ac", "U_SIA", "V_SIA", "D_SIA")))
         ps, _z = _params_struct(params)
@@ -405,7 +494,7 @@ class DeviceMesh:
         nZ = len(params["zeta"])
         A = None if A_flow is None else np.asfortranarray(A_flow, dtype=np.float64)
         d = np.ascontiguousarray(dHb_dt, dtype=np.float64)
-        outs = [np.zeros((self.nV, nZ), order="F") for _ in range(3)]
+        outs = [_pool.array((self.nV, nZ), order="F") for _ in range(3)]
         so = nat.Sia3dOut(*(o.ctypes.data for o in outs))
         ps, _z = _params_struct(params)
         rc = L.ufe_sia3d_solve(self._h, ct.byref(ps), _ptr(A), d.ctypes.data, ct.byref(so))
@@ -428,7 +517,7 @@ class DeviceMesh:
             keys += ["Ti_pmp", "Cpi", "Ki"]
         if flow_law == nat.UFE_FLOW_ARRHENIUS:
             keys.append("Ti_Ac")
-        out = {k: np.zeros(shapes[k], order="F") for k in keys}
+        out = {k: _pool.array(shapes[k], order="F") for k in keys}
         po = nat.PhyspropOut(*(_ptr(out.get(k)) for k in nat.PHYSPROP_OUT_FIELDS))
         T = None if Ti is None else np.asfortranarray(Ti, dtype=np.float64)
         if T is not None and T.shape != (self.nV, nZ):
@@ -463,8 +552,8 @@ class DeviceMesh:
         for a in arrs:
             if a is not None and a.shape != (self.nV, nZ):
                 raise ValueError("fields must be (nV, nZ)")
-        ddx = np.zeros((self.nV, nZ), order="F")
-        ddy = np.zeros((self.nV, nZ), order="F")
+        ddx = _pool.array((self.nV, nZ), order="F")
+        ddy = _pool.array((self.nV, nZ), order="F")
         miss = ct.c_int64(0)
         ps, _z = _params_struct(params)
         rc = L.ufe_upwind_derivatives_3d(self._h, ct.byref(ps), *(_ptr(a) for a in arrs), ddx.ctypes.data,
@@ -486,9 +575,10 @@ class DeviceMesh:
         ti = nat.ThicknessIn(_ptr(keep["A"]), _ptr(keep["Cw"]), _ptr(keep["usia"]), _ptr(keep["ussa"]),
                              _ptr(keep["SMB"]), _ptr(keep["BMB"]), _ptr(keep["noice"]), float(dt),
                              1 if zero_edges else 0)
-        H = np.array(Hi, dtype=np.float64, copy=True)
-        out = dict(Hi_prev=np.zeros(self.nV), dHi_dt=np.zeros(self.nV),
-                   dVi_in=np.zeros(keep["Cw"].shape, order="F"))
+        H = _pool.array(np.shape(Hi))
+        H[...] = Hi
+        out = dict(Hi_prev=_pool.array(self.nV), dHi_dt=_pool.array(self.nV),
+                   dVi_in=_pool.array(keep["Cw"].shape, order="F"))
         to = nat.ThicknessOut(*(out[k].ctypes.data for k in ("Hi_prev", "dHi_dt", "dVi_in")))
         rc = L.ufe_thickness_update(self._h, ct.byref(ti), H.ctypes.data, ct.byref(to))
         if rc != nat.UFE_OK:
@@ -505,11 +595,11 @@ class DeviceMesh:
         keep["A_flow_Ac"] = np.asfortranarray(fields["A_flow_Ac"], dtype=np.float64)
         si = nat.SiaIn(*(keep[k].ctypes.data for k in ("mask_sheet_Ac", "Hi_Ac", "dHs_dx_Ac", "dHs_dy_Ac",
                                                         "dHs_dp_Ac", "dHs_do_Ac", "A_flow_Ac")))
-        out = dict(D_SIA_3D_Ac=np.zeros((self.nAc, nZ), order="F") if want_3d else None)
+        out = dict(D_SIA_3D_Ac=_pool.array((self.nAc, nZ), order="F") if want_3d else None)
         for k in ("D_SIA_Ac", "Ux_SIA_Ac", "Uy_SIA_Ac", "Up_SIA_Ac", "Uo_SIA_Ac"):
-            out[k] = np.zeros(self.nAc)
+            out[k] = _pool.array(self.nAc)
         for k in ("U_SIA", "V_SIA", "D_SIA"):
-            out[k] = np.zeros(self.nV)
+            out[k] = _pool.array(self.nV)
         so = nat.SiaOut(*(_ptr(out[k]) for k in ("D_SIA_3D_Ac", "D_SIA_Ac", "Ux_SIA_Ac", "Uy_SIA_Ac", "Up_SIA_Ac",
                                                   "Uo_SIA_Ac", "U_SIA", "V_SIA", "D_SIA")))
         ps, _z = _params_struct(params)
@@ -600,6 +690,7 @@ class Batch:
         if getattr(self, "_h", None):
             nat.load().ufe_batch_destroy(self._h)
             self._h = None
+            _pool.release()
 
     def __del__(self):
         try:
