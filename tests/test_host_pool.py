@@ -43,7 +43,11 @@ def test_idle_memory_is_bounded_and_released():
     del arrays
     gc.collect()
     assert 0 < pool._bytes <= 1 << 20
+    held = pool.array(65536)
     pool.release()
+    assert pool._bytes == 0 and not pool._idle
+    del held   # leased before the release: not kept
+    gc.collect()
     assert pool._bytes == 0 and not pool._idle
 
 

@@ -27,14 +27,15 @@ class _HostPool:
     6 us per MB for the copy from the device), so blocks of a page or more are handed out again
     once no array or view uses them. A block belongs to the array it backs until that array, and
     every view of it, is gone (the lease is the array's buffer). At most ``limit`` idle bytes are
-    kept; blocks beyond that, and all idle ones on ``release`` (when a mesh or a batch is closed),
-    go back to the allocator. Safe with several threads.
+    kept; blocks beyond that, and on ``release`` (when a mesh or a batch is closed) all idle ones and
+    those then in use once they are dropped, go back to the allocator. Safe with several threads.
     """
 
     def __init__(self, limit: int = 512 << 20, smallest: int = 64 << 10):
         self.limit, self.smallest = limit, smallest
         self._idle: dict = {}
         self._bytes = 0
+        self._age = 0   # releases so far: a block leased before one is not kept when it comes back
         self._lock = threading.RLock()   # a lease may end (in a collection) while its thread holds the lock
 
     def array(self, shape, dtype=np.float64, order: str = "C"):
@@ -50,18 +51,38 @@ class _HostPool:
             block = blocks.pop() if blocks else None
             if block is not None:
                 self._bytes -= size
+            age = self._age
         if block is None:
             block = np.empty(size, np.uint8)
-        return np.frombuffer(_Lease(self, block), dtype, nbytes // dtype.itemsize).reshape(shape, order=order)
+        return np.frombuffer(_Lease(self, block, age), dtype, nbytes // dtype.itemsize).reshape(shape, order=order)
+
+    def group(self, shapes, dtype=np.float64, order: str = "C", most: int = 16 << 20):
+        """Uninitialised arrays of the given shapes, one after the other in blocks of at most ``most``
+        bytes (where one array is no larger): results in the order in which the library keeps them on
+        the device come back in few copies. Larger blocks the allocator would take fresh from the
+        system each time."""
+        shapes = [(s,) if np.isscalar(s) else tuple(s) for s in shapes]
+        sizes = [int(np.prod(s, dtype=np.int64)) for s in shapes]
+        out, i, limit = [], 0, most // np.dtype(dtype).itemsize
+        while i < len(sizes):
+            n, k = sizes[i], i + 1
+            while k < len(sizes) and n + sizes[k] <= limit:
+                n, k = n + sizes[k], k + 1
+            flat, at = self.array(n, dtype), 0
+            for shape, size in zip(shapes[i:k], sizes[i:k]):
+                out.append(flat[at:at + size].reshape(shape, order=order))
+                at += size
+            i = k
+        return out
 
     def zeros(self, shape, dtype=np.float64, order: str = "C"):
         a = self.array(shape, dtype, order)
         a.fill(0)
         return a
 
-    def give_back(self, block):
+    def give_back(self, block, age):
         with self._lock:
-            if self._bytes + block.size <= self.limit:
+            if age == self._age and self._bytes + block.size <= self.limit:
                 self._idle.setdefault(block.size, []).append(block)
                 self._bytes += block.size
 
@@ -69,19 +90,20 @@ class _HostPool:
         with self._lock:
             self._idle.clear()
             self._bytes = 0
+            self._age += 1
 
 
 class _Lease:
     """One array's use of a pool block (the buffer that the array is made from)."""
 
-    def __init__(self, pool, block):
-        self._pool, self._block = pool, block
+    def __init__(self, pool, block, age):
+        self._pool, self._block, self._age = pool, block, age
 
     def __buffer__(self, flags):
         return memoryview(self._block)
 
     def __del__(self):
-        self._pool.give_back(self._block)
+        self._pool.give_back(self._block, self._age)
 
 
 _pool = _HostPool()
@@ -253,10 +275,11 @@ def _ssa_structs(nV, nAc, nA, fields: dict, warm: dict | None):
 
 
 def _download_structs(nV, nAc, nA):
-    io = {k: _pool.array(nV) for k in ("U_SSA", "V_SSA")}
-    io.update({k: _pool.array(nAc) for k in ("Ux_SSA_Ac", "Uy_SSA_Ac", "Up_SSA_Ac", "Uo_SSA_Ac")})
-    # zero: not written after the early-out of a solve without grounded ice
-    io.update({k: _pool.zeros(nA) for k in ("N_AaAc", "eta_AaAc", "S_AaAc", "tau_c_AaAc", "phi_fric_AaAc")})
+    names = ("U_SSA", "V_SSA", "Ux_SSA_Ac", "Uy_SSA_Ac", "Up_SSA_Ac", "Uo_SSA_Ac", "N_AaAc", "eta_AaAc", "S_AaAc",
+             "tau_c_AaAc", "phi_fric_AaAc")
+    io = dict(zip(names, _pool.group([nV] * 2 + [nAc] * 4 + [nA] * 5)))
+    for k in names[6:]:   # not written after the early-out of a solve without grounded ice
+        io[k].fill(0)
     sio = nat.SsaInout(*(io[k].ctypes.data for k in ("U_SSA", "V_SSA", "Ux_SSA_Ac", "Uy_SSA_Ac", "N_AaAc")))
     so = nat.SsaOut(*(io[k].ctypes.data for k in ("Up_SSA_Ac", "Uo_SSA_Ac", "eta_AaAc", "S_AaAc", "tau_c_AaAc",
                                                    "phi_fric_AaAc")))
@@ -315,8 +338,7 @@ class DeviceMesh:
         L = nat.load()
         if buffers is None:
             si, sio, io, keep = self._ssa_structs(fields, warm)
-            out = {k: _pool.array(self.nAc) for k in ("Up_SSA_Ac", "Uo_SSA_Ac")}
-            out.update({k: _pool.array(self.nVAaAc) for k in ("eta_AaAc", "S_AaAc", "tau_c_AaAc", "phi_fric_AaAc")})
+            out = dict(zip(SSA_OUT_FIELDS, _pool.group([self.nAc] * 2 + [self.nVAaAc] * 4)))
         else:
             if warm is not None:
                 raise ValueError("with buffers the warm start is the buffers' content")
@@ -430,10 +452,10 @@ class DeviceMesh:
         L = nat.load()
         ints = {"mask_ocean", "mask_ice", "mask_sheet", "mask_shelf", "mask_ocean_Ac", "mask_ice_Ac", "mask_sheet_Ac",
                 "mask_shelf_Ac", "mask_gl_Ac"}
-        out = {}
-        for k in nat.GEOM_OUT_FIELDS:
-            n = self.nAc if k.endswith("_Ac") else self.nV
-            out[k] = _pool.array(n, dtype=np.int32 if k in ints else np.float64)
+        size = lambda k: self.nAc if k.endswith("_Ac") else self.nV  # noqa: E731
+        out = dict.fromkeys(nat.GEOM_OUT_FIELDS)
+        for dtype, names in ((np.float64, [k for k in out if k not in ints]), (np.int32, [k for k in out if k in ints])):
+            out.update(zip(names, _pool.group([size(k) for k in names], dtype)))
         go = nat.GeometryOut(*(out[k].ctypes.data for k in nat.GEOM_OUT_FIELDS))
         arrs = [np.ascontiguousarray(a, dtype=np.float64) for a in (Hi, Hb, SL)]
         rc = L.ufe_geometry_update(self._h, *(a.ctypes.data for a in arrs), ct.byref(go))
@@ -446,7 +468,8 @@ class DeviceMesh:
         mask_<name> (nV) and mask_<name>_Ac (nAc) for each of nat.MASK_NAMES, plus the type
         masks mask (nV) and mask_Ac (nAc)."""
         L = nat.load()
-        out = {k: _pool.array(self.nAc if k.endswith("_Ac") else self.nV, dtype=np.int32) for k in nat.MASK_OUT_FIELDS}
+        out = dict(zip(nat.MASK_OUT_FIELDS, _pool.group(
+            [self.nAc if k.endswith("_Ac") else self.nV for k in nat.MASK_OUT_FIELDS], np.int32)))
         mo = nat.MaskOut(*(out[k].ctypes.data for k in nat.MASK_OUT_FIELDS))
         rc = L.ufe_geometry_masks(self._h, ct.byref(mo))
         if rc != nat.UFE_OK:
@@ -474,11 +497,7 @@ class DeviceMesh:
         L = nat.load()
         nZ = len(params["zeta"])
         A = None if A_flow_Ac is None else np.asfortranarray(A_flow_Ac, dtype=np.float64)
-        out = dict(D_SIA_3D_Ac=_pool.array((self.nAc, nZ), order="F"))
-        for k in ("D_SIA_Ac", "Ux_SIA_Ac", "Uy_SIA_Ac", "Up_SIA_Ac", "Uo_SIA_Ac"):
-            out[k] = _pool.array(self.nAc)
-        for k in ("U_SIA", "V_SIA", "D_SIA"):
-            out[k] = _pool.array(self.nV)
+        out = self._sia_out(nZ)
         so = nat.SiaOut(*(_ptr(out[k]) for k in ("D_SIA_3D_Ac", "D_SIA_Ac", "Ux_SIA_Ac", "Uy_SIA_Ac", "Up_SIA_Ac",
                                                   "Uo_SIA_Ac", "U_SIA", "V_SIA", "D_SIA")))
         ps, _z = _params_struct(params)
@@ -494,7 +513,7 @@ class DeviceMesh:
         nZ = len(params["zeta"])
         A = None if A_flow is None else np.asfortranarray(A_flow, dtype=np.float64)
         d = np.ascontiguousarray(dHb_dt, dtype=np.float64)
-        outs = [_pool.array((self.nV, nZ), order="F") for _ in range(3)]
+        outs = _pool.group([(self.nV, nZ)] * 3, order="F")
         so = nat.Sia3dOut(*(o.ctypes.data for o in outs))
         ps, _z = _params_struct(params)
         rc = L.ufe_sia3d_solve(self._h, ct.byref(ps), _ptr(A), d.ctypes.data, ct.byref(so))
@@ -517,7 +536,8 @@ class DeviceMesh:
             keys += ["Ti_pmp", "Cpi", "Ki"]
         if flow_law == nat.UFE_FLOW_ARRHENIUS:
             keys.append("Ti_Ac")
-        out = {k: _pool.array(shapes[k], order="F") for k in keys}
+        keys.sort(key=("A_flow", "Ti_pmp", "Cpi", "Ki", "A_flow_Ac", "Ti_Ac", "A_flow_mean", "A_flow_mean_Ac").index)
+        out = dict(zip(keys, _pool.group([shapes[k] for k in keys], order="F")))
         po = nat.PhyspropOut(*(_ptr(out.get(k)) for k in nat.PHYSPROP_OUT_FIELDS))
         T = None if Ti is None else np.asfortranarray(Ti, dtype=np.float64)
         if T is not None and T.shape != (self.nV, nZ):
@@ -552,8 +572,7 @@ class DeviceMesh:
         for a in arrs:
             if a is not None and a.shape != (self.nV, nZ):
                 raise ValueError("fields must be (nV, nZ)")
-        ddx = _pool.array((self.nV, nZ), order="F")
-        ddy = _pool.array((self.nV, nZ), order="F")
+        ddx, ddy = _pool.group([(self.nV, nZ)] * 2, order="F")
         miss = ct.c_int64(0)
         ps, _z = _params_struct(params)
         rc = L.ufe_upwind_derivatives_3d(self._h, ct.byref(ps), *(_ptr(a) for a in arrs), ddx.ctypes.data,
@@ -575,10 +594,9 @@ class DeviceMesh:
         ti = nat.ThicknessIn(_ptr(keep["A"]), _ptr(keep["Cw"]), _ptr(keep["usia"]), _ptr(keep["ussa"]),
                              _ptr(keep["SMB"]), _ptr(keep["BMB"]), _ptr(keep["noice"]), float(dt),
                              1 if zero_edges else 0)
-        H = _pool.array(np.shape(Hi))
+        flux, H, prev, rate = _pool.group([keep["Cw"].shape, np.shape(Hi), self.nV, self.nV], order="F")
         H[...] = Hi
-        out = dict(Hi_prev=_pool.array(self.nV), dHi_dt=_pool.array(self.nV),
-                   dVi_in=_pool.array(keep["Cw"].shape, order="F"))
+        out = dict(Hi_prev=prev, dHi_dt=rate, dVi_in=flux)
         to = nat.ThicknessOut(*(out[k].ctypes.data for k in ("Hi_prev", "dHi_dt", "dVi_in")))
         rc = L.ufe_thickness_update(self._h, ct.byref(ti), H.ctypes.data, ct.byref(to))
         if rc != nat.UFE_OK:
@@ -586,6 +604,13 @@ class DeviceMesh:
         return H, out["Hi_prev"], out["dHi_dt"], out["dVi_in"]
 
     # ---------------------------------------------------------------- SIA
+    def _sia_out(self, nZ: int, want_3d: bool = True) -> dict:
+        names = ("D_SIA_3D_Ac", "D_SIA_Ac", "Ux_SIA_Ac", "Uy_SIA_Ac", "Up_SIA_Ac", "Uo_SIA_Ac", "U_SIA", "V_SIA", "D_SIA")
+        shapes = [(self.nAc, nZ)] + [self.nAc] * 5 + [self.nV] * 3
+        if not want_3d:
+            return dict(zip(names, [None] + _pool.group(shapes[1:], order="F")))
+        return dict(zip(names, _pool.group(shapes, order="F")))
+
     def solve_sia(self, fields: dict, params: dict, want_3d: bool = True):
         L = nat.load()
         nZ = len(params["zeta"])
@@ -595,11 +620,7 @@ class DeviceMesh:
         keep["A_flow_Ac"] = np.asfortranarray(fields["A_flow_Ac"], dtype=np.float64)
         si = nat.SiaIn(*(keep[k].ctypes.data for k in ("mask_sheet_Ac", "Hi_Ac", "dHs_dx_Ac", "dHs_dy_Ac",
                                                         "dHs_dp_Ac", "dHs_do_Ac", "A_flow_Ac")))
-        out = dict(D_SIA_3D_Ac=_pool.array((self.nAc, nZ), order="F") if want_3d else None)
-        for k in ("D_SIA_Ac", "Ux_SIA_Ac", "Uy_SIA_Ac", "Up_SIA_Ac", "Uo_SIA_Ac"):
-            out[k] = _pool.array(self.nAc)
-        for k in ("U_SIA", "V_SIA", "D_SIA"):
-            out[k] = _pool.array(self.nV)
+        out = self._sia_out(nZ, want_3d)
         so = nat.SiaOut(*(_ptr(out[k]) for k in ("D_SIA_3D_Ac", "D_SIA_Ac", "Ux_SIA_Ac", "Uy_SIA_Ac", "Up_SIA_Ac",
                                                   "Uo_SIA_Ac", "U_SIA", "V_SIA", "D_SIA")))
         ps, _z = _params_struct(params)

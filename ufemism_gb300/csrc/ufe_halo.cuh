@@ -318,17 +318,6 @@ template <> struct Prog<kMixed> {
   }
 };
 
-// a / b rounded to nearest, given r = 1 / b rounded to nearest (Markstein, IBM J. Res. Dev. 34,
-// 1990: the quotient corrected once by its exact remainder is the correctly rounded one when
-// nothing over- or underflows). Other exponents take the division itself. GB300's FP64 pipe
-// makes the division the costliest step of the parity mode's update.
-__device__ __forceinline__ double divide_by(double a, double b, double r) {
-  const double q = a * r;
-  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eq = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
-  if (ea - 200u < 1600u && eq - 200u < 1600u) return fma(fma(-q, b, a), r, q);
-  return a / b;
-}
-
 // FP64 sweeps (as phase_sweep_fast and phase_sweep_exact). An FP64 instruction occupies a quarter
 // SM's unit for 64 cycles (measured), so what counts is how many a warp issues in a row: a lane
 // updates one component of one row (16 rows a unit, two units a slice; lanes 0-15 U, 16-31 V),

@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include "../../include/ufemism_gb300.h"
 
@@ -178,6 +179,48 @@ struct ufe_mesh_s {
 };
 
 namespace ufe {
+// Copies from the device to the caller's arrays, queued on a stream; ranges that continue the one
+// before on both sides are one copy (each costs about 20 us from the queue, 80 MB only 460 us).
+// A null destination is skipped.
+class CopyOut {
+ public:
+  CopyOut(cudaStream_t s, const char *what) : s_(s), what_(what) {}
+  template <class T>
+  void add(T *dst, const T *src, size_t n) {
+    if (!dst || rc_ || n == 0) return;
+    const Range r{reinterpret_cast<char *>(dst), reinterpret_cast<const char *>(src), n * sizeof(T)};
+    if (!run_.empty() && (r.dst != run_.back().dst + run_.back().bytes || r.src != run_.back().src + run_.back().bytes)) flush();
+    run_.push_back(r);
+  }
+  int flush() {
+    if (!run_.empty() && !rc_) {
+      size_t total = 0;
+      for (const Range &r : run_) total += r.bytes;
+      cudaError_t e = cudaMemcpyAsync(run_[0].dst, run_[0].src, total, cudaMemcpyDeviceToHost, s_);
+      if (e == cudaErrorInvalidValue && run_.size() > 1) {   // neighbours that were page-locked separately
+        cudaGetLastError();
+        e = cudaSuccess;
+        for (const Range &r : run_)
+          if (e == cudaSuccess) e = cudaMemcpyAsync(r.dst, r.src, r.bytes, cudaMemcpyDeviceToHost, s_);
+      }
+      rc_ = cuda_status(e, what_);
+    }
+    run_.clear();
+    return rc_;
+  }
+
+ private:
+  struct Range {
+    char *dst;
+    const char *src;
+    size_t bytes;
+  };
+  cudaStream_t s_;
+  const char *what_;
+  std::vector<Range> run_;
+  int rc_ = 0;
+};
+
 void ssa_free(SsaWork *w);
 void sia_free(SiaWork *w);
 void adj_free(AdjWork *w);
@@ -192,4 +235,43 @@ const double *sia_device_Up(ufe_mesh_h h);
 // ufe_ssa_upload from device arrays of this device (sheet_count: grounded-ice vertices).
 int ssa_upload_impl(ufe_mesh_h h, const ufe_params *p, const ufe_ssa_in *in, const ufe_ssa_inout *io,
                     bool in_on_device, long long sheet_count);
+
+#ifdef __CUDACC__
+// a / b rounded to nearest, given r = 1 / b rounded to nearest (Markstein, IBM J. Res. Dev. 34,
+// 1990: the quotient corrected once by its exact remainder is the correctly rounded one when
+// nothing over- or underflows). Other exponents take the division itself. GB300's FP64 pipe
+// (64 cycles a warp instruction on a quarter SM) makes a division cost about 20 of them, this 3.
+static __device__ __noinline__ double divide_ieee(double a, double b) { return a / b; }   // kept off the common path
+
+__device__ __forceinline__ double divide_by(double a, double b, double r) {
+  const double q = a * r;
+  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eq = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
+  if (ea - 200u < 1600u && eq - 200u < 1600u) return fma(fma(-q, b, a), r, q);
+  if (((unsigned long long)__double_as_longlong(a) << 1) == 0ull) return q;   // a zero: exact
+  return divide_ieee(a, b);
+}
+
+// 1 / b to within a unit in the last place for normal b: two Newton steps (y += y (1 - b y)) from the
+// hardware's 20-bit estimate, 4 FP64 instructions.
+__device__ __forceinline__ double reciprocal_newton(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  y = fma(y, fma(-b, y, 1.0), y);
+  return fma(y, fma(-b, y, 1.0), y);
+}
+
+// 1 / n of the small counts that the kernels divide by, rounded to nearest (a kernel parameter).
+struct CountReciprocals {
+  double n[kMaxDeg + 1], r[kMaxDeg + 1];   // n as a double, and 1 / n
+};
+inline CountReciprocals count_reciprocals() {
+  CountReciprocals c;
+  c.n[0] = c.r[0] = 0.0;
+  for (int n = 1; n <= kMaxDeg; ++n) {
+    c.n[n] = (double)n;
+    c.r[n] = 1.0 / (double)n;
+  }
+  return c;
+}
+#endif
 }  // namespace ufe

@@ -2333,23 +2333,25 @@ extern "C" int ufe_ssa_download(ufe_mesh_h h, ufe_ssa_inout *io, ufe_ssa_out *ou
   const size_t nV = w->nV, nAc = w->nAc, nA = w->nA;
   cudaStream_t s = h->stream;
   const double *so = w->stage_out;
-  int rc = d2h(io->U_SSA, so, nV, s);
-  if (!rc) rc = d2h(io->V_SSA, so + nV, nV, s);
-  if (!rc) rc = d2h(io->Ux_SSA_Ac, so + 2 * nV, nAc, s);
-  if (!rc) rc = d2h(io->Uy_SSA_Ac, so + 2 * nV + nAc, nAc, s);
+  CopyOut back(s, "D2H");   // in the staging buffer's order
+  back.add(io->U_SSA, so, nV);
+  back.add(io->V_SSA, so + nV, nV);
+  back.add(io->Ux_SSA_Ac, so + 2 * nV, nAc);
+  back.add(io->Uy_SSA_Ac, so + 2 * nV + nAc, nAc);
   const double *acb = so + 2 * nV + 2 * nAc;
   if (out) {
-    if (!rc) rc = d2h(out->Up_SSA_Ac, acb, nAc, s);
-    if (!rc) rc = d2h(out->Uo_SSA_Ac, acb + nAc, nAc, s);
+    back.add(out->Up_SSA_Ac, acb, nAc);
+    back.add(out->Uo_SSA_Ac, acb + nAc, nAc);
   }
   const double *ab = acb + 2 * nAc;
-  if (!rc && io->N_AaAc && !w->zero) rc = d2h(io->N_AaAc, ab, nA, s);
+  if (!w->zero) back.add(io->N_AaAc, ab, nA);
   if (out && !w->zero) {
-    if (!rc) rc = d2h(out->eta_AaAc, ab + nA, nA, s);
-    if (!rc) rc = d2h(out->S_AaAc, ab + 2 * nA, nA, s);
-    if (!rc) rc = d2h(out->tau_c_AaAc, ab + 3 * nA, nA, s);
-    if (!rc) rc = d2h(out->phi_fric_AaAc, ab + 4 * nA, nA, s);
+    back.add(out->eta_AaAc, ab + nA, nA);
+    back.add(out->S_AaAc, ab + 2 * nA, nA);
+    back.add(out->tau_c_AaAc, ab + 3 * nA, nA);
+    back.add(out->phi_fric_AaAc, ab + 4 * nA, nA);
   }
+  int rc = back.flush();
   if (!rc) rc = cuda_status(cudaStreamSynchronize(s), "ssa download");
   return rc;
 }
