@@ -393,15 +393,15 @@ int ufe_ssa_vjp(ufe_mesh_h mesh, const ufe_params *params, const ufe_vjp_params 
  * each class gets CTAs in proportion to its estimated work. With use_graph the whole batch
  * (gathers, the persistent solve, scatters) is captured once per parameter set and upload
  * state and replayed as a CUDA graph. Members share one ufe_params; their inputs are
- * uploaded one by one (the arrays of ufe_ssa_upload). In the mixed precision the members run
- * the halo sweeps of the single solves when the largest member's working copy fits beside the
- * CTAs the plan keeps resident (else the phased sweeps); either gives each member the result of
- * its single solve. */
+ * uploaded one by one (the arrays of ufe_ssa_upload). The members run the halo sweeps of the
+ * single solves when the largest member's working copy fits beside the CTAs the plan keeps
+ * resident (else the phased sweeps); either gives each member the result of its single solve. */
 typedef struct ufe_batch_s *ufe_batch_h;
 typedef struct ufe_batch_config {
   int32_t team_ctas;     /* > 0: every member solved by a team of this many CTAs */
   int32_t rows_per_cta;  /* team_ctas == 0: member team = the power of two nearest above
-                            rows / rows_per_cta (0: 8192 rows) - the per-CTA packing */
+                            rows / rows_per_cta - the per-CTA packing (0: 8192 rows, and CTAs that
+                            all members at once leave idle go to those expected to take longest) */
   int32_t block;         /* threads per CTA: 1024, 512 or 256 (0: 1024); 512 and 256 run 2 and 4 CTAs per SM */
   int32_t use_graph;     /* 1: capture and replay the batch as a CUDA graph */
 } ufe_batch_config;

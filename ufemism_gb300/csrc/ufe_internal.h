@@ -147,6 +147,7 @@ struct DevMesh {
   int max_halo = 0;             // largest number of halo rows of a patch
   int max_hslices = 0;          // largest number of program slices of a patch
   int n_hslices = 0;
+  size_t max_hprog32 = 0, max_hprog64 = 0;   // bytes of the largest patch's blocks
   int n_export = 0;             // rows that are another patch's halo rows
   int *hp_slice = nullptr;      // [n_patch * 7 + 1] first program slice of phases 0..6 of each patch, then the end
   int *hp_split = nullptr;      // [n_patch] first slice of phase 0's rows that read halo slots (the others come first)

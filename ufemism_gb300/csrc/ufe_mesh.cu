@@ -494,6 +494,7 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
       // (bank_aware_slices: by degree, lanes chosen to spread the working-copy gathers over
       // the shared-memory banks)
       const int first_slice = (int)hslice_e0.size();
+      const size_t first32 = hprog32.size(), first64 = hprog64.size();
       for (int f = 0; f < 7; ++f) {
         hp_slice.push_back((int)hslice_e0.size());
         std::vector<int> rows;   // device rows, -1 = padding slot
@@ -593,6 +594,8 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
         }
       }
       m.max_hslices = std::max(m.max_hslices, (int)hslice_e0.size() - first_slice);
+      m.max_hprog32 = std::max(m.max_hprog32, hprog32.size() - first32);
+      m.max_hprog64 = std::max(m.max_hprog64, hprog64.size() - first64);
       if (m.max_hslices > kMaxPatchSlices || nE_h >= ((int64_t)1 << 31) ||
           hprog64.size() / 16 >= ((size_t)1 << 31)) halo_ok = false;
     }

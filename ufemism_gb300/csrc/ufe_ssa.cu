@@ -2437,6 +2437,31 @@ double member_work(int rows, int T, int block) {
   return (double)T * sweeps * per_sweep_us;
 }
 
+// With the default packing: CTAs that are left when every member has its team at once go to the
+// members expected to take longest (a batch ends with its slowest member), a team growing by the
+// sizes 1, 2, 3, 4, 6, 8, 12, ... The estimate of a solve: rows^0.75 sweeps (184, 324, 876 and 3129
+// on domes of 284, 996, 3336 and 15984 vertices), each 3.4 us and 1 us per 700 rows of a CTA
+// (mixed; 12.1 us at 5,400 rows plus their halo).
+void spread_teams(const int32_t *rows, int n, int resident, int32_t *team) {
+  auto next = [](int t) { return (t & (t - 1)) == 0 ? (t < 2 ? t + 1 : t / 2 * 3) : t / 3 * 4; };
+  auto time = [&](int m) { return std::pow((double)rows[m], 0.75) * (3.4 + (double)rows[m] / team[m] / 700.0); };
+  int used = 0;
+  for (int m = 0; m < n; ++m) used += team[m];
+  if (used >= resident) return;
+  std::vector<char> done(n, 0);
+  for (;;) {
+    int worst = -1;
+    for (int m = 0; m < n; ++m)
+      if (!done[m] && (worst < 0 || time(m) > time(worst))) worst = m;
+    if (worst < 0) return;
+    const int t = next(team[worst]);
+    // teams of at least 128 rows a CTA; at most half the CTAs (the planner fits one team of every class)
+    if (t > rows[worst] / 128 || 2 * t > resident + 1 || used + t - team[worst] > resident) { done[worst] = 1; continue; }
+    used += t - team[worst];
+    team[worst] = t;
+  }
+}
+
 int plan_batch(const int32_t *rows, int n, const ufe_batch_config &cfg, int resident, int32_t *team_of_member,
                ufe_batch_plan_out *plan) {
   const int block = cfg.block ? cfg.block : 1024;
@@ -2465,6 +2490,7 @@ int plan_batch(const int32_t *rows, int n, const ufe_batch_config &cfg, int resi
     }
     team_of_member[m] = T;
   }
+  if (cfg.team_ctas == 0 && cfg.rows_per_cta == 0) spread_teams(rows, n, resident, team_of_member);
   // Classes: distinct team sizes, largest first.
   std::vector<int> sizes(team_of_member, team_of_member + n);
   std::sort(sizes.begin(), sizes.end(), std::greater<int>());
@@ -2525,11 +2551,14 @@ struct ufe_batch_s {
   int n = 0;                          // members
   int block = 0;                      // threads per CTA of the batched kernel
   bool use_graph = true;
-  // mixed members on the halo sweeps: every member has the program and the largest working copy
-  // (plus halo indices) fits the CTAs the plan keeps resident
-  bool halo_ok = false;
-  int halo_index_off = 0, halo_stage_off = 0;
-  size_t halo_smem = 0;
+  // members on the halo sweeps, per SweepMode: every member has the program and the largest working
+  // copy (plus halo indices) fits the CTAs the plan keeps resident; what is left of the shared
+  // memory holds program slices
+  struct Halo {
+    bool ok = false;
+    int index_off = 0, stage_off = 0, stage_bytes = 0;
+    size_t smem = 0;
+  } halo[3];
   ufe_batch_plan_out plan{};
   int n_teams = 0;
   std::vector<int32_t> team_of_member;
@@ -2573,11 +2602,15 @@ void batch_free(ufe_batch_s *b) {
   delete b;
 }
 
-// The batched kernel for a sweep mode and CTA shape (nullptr: not built); halo: the mixed
-// members' halo sweeps, which run half the threads with twice the registers (see kHaloBlock).
+// The batched kernel for a sweep mode and CTA shape (nullptr: not built); halo: the members' halo
+// sweeps, which run half the threads with twice the registers (see kHaloBlock).
 const void *batched_kernel(int mode, int block, bool halo = false) {
   if (halo) {
     switch (mode * 10000 + block) {
+      case kExact64 * 10000 + 1024: return (const void *)ssa_batched<kExact64, 512, 1, true>;
+      case kFast64 * 10000 + 1024: return (const void *)ssa_batched<kFast64, 512, 1, true>;
+      case kFast64 * 10000 + 512: return (const void *)ssa_batched<kFast64, 256, 2, true>;
+      case kFast64 * 10000 + 256: return (const void *)ssa_batched<kFast64, 128, 4, true>;
       case kMixed * 10000 + 1024: return (const void *)ssa_batched<kMixed, 512, 1, true>;
       case kMixed * 10000 + 512: return (const void *)ssa_batched<kMixed, 256, 2, true>;
       case kMixed * 10000 + 256: return (const void *)ssa_batched<kMixed, 128, 4, true>;
@@ -2668,10 +2701,10 @@ int batch_enqueue(ufe_batch_s *b, const ufe_params *p, int mode) {
     bool solve = false;
     SsaArgs a;
     rc = launch_prepare(b->members[m], p, s, &a, &solve);
-    if (!rc && solve && mode == kMixed && b->halo_ok) {
-      a.halo_index_off = b->halo_index_off;
-      a.stage_off = b->halo_stage_off;
-      a.stage_bytes = 0;
+    if (!rc && solve && b->halo[mode].ok) {
+      a.halo_index_off = b->halo[mode].index_off;
+      a.stage_off = b->halo[mode].stage_off;
+      a.stage_bytes = b->halo[mode].stage_bytes;
       rc = prepare_halo(b->members[m], mode, s, &a);
     }
     if (!rc && solve) {
@@ -2712,13 +2745,13 @@ int batch_enqueue(ufe_batch_s *b, const ufe_params *p, int mode) {
     ba.team_of_cta = tcd; ba.team_info = tid; ba.class_range = reinterpret_cast<const int2 *>(tid + b->n_teams);
     ba.queue = queue; ba.team_bar = team_bar; ba.team_member = team_member;
     ba.times = b->times_dev; ba.err = b->err_dev; ba.timeout_ns = wait_timeout_ns();
-    const bool halo = mode == kMixed && b->halo_ok;
+    const bool halo = b->halo[mode].ok;
     if (halo) fn = batched_kernel(mode, b->block, true);
     if (!rc) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)pl.grid_ctas);
       cfg.blockDim = dim3((unsigned)(halo ? b->block / 2 : b->block));
-      cfg.dynamicSmemBytes = halo ? b->halo_smem : 0;
+      cfg.dynamicSmemBytes = halo ? b->halo[mode].smem : 0;
       cfg.stream = s;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeCooperative;
@@ -2800,8 +2833,8 @@ extern "C" int ufe_batch_create(const ufe_mesh_desc *descs, int32_t n, const ufe
     if (!rc) b->cost[k] = member_work(rows[k], 1, 1024);
   }
   if (!rc) {
-    // Mixed members run the halo sweeps when every member has the program and the largest working
-    // copy with its halo indices leaves the plan's CTAs co-resident (else the phased sweeps).
+    // Members run the halo sweeps when every member has the program and the largest working copy
+    // with its halo indices leaves the plan's CTAs co-resident (else the phased sweeps).
     int max_local = 0, max_halo = 0;
     bool all = true;
     for (ufe_mesh_h h : b->members) {
@@ -2809,20 +2842,45 @@ extern "C" int ufe_batch_create(const ufe_mesh_desc *descs, int32_t n, const ufe
       max_local = std::max(max_local, h->m.max_local);
       max_halo = std::max(max_halo, h->m.max_halo);
     }
-    const void *fn = batched_kernel(kMixed, block, true);
-    if (all && fn) {
-      const size_t idx_off = ((size_t)max_local + 1) * sizeof(float2);
+    for (int mode = 0; mode < 3 && all; ++mode) {
+      const void *fn = batched_kernel(mode, block, true);
+      if (!fn) continue;
+      ufe_batch_s::Halo &q = b->halo[mode];
+      const size_t elem = mode == kMixed ? sizeof(float2) : sizeof(double2);
+      const size_t idx_off = ((size_t)max_local + 1) * elem;
       const size_t stage_off = (idx_off + (size_t)max_halo * sizeof(int) + 15) / 16 * 16;
-      int per_sm = 0;
-      if (raise_dynamic_smem(fn, b->device, stage_off) &&
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block / 2, stage_off) == cudaSuccess &&
-          per_sm * b->num_sms >= b->plan.grid_ctas) {
-        b->halo_ok = true;
-        b->halo_index_off = (int)idx_off;
-        b->halo_stage_off = (int)stage_off;
-        b->halo_smem = stage_off;
+      auto fits = [&](size_t bytes) {
+        int per_sm = 0;
+        const bool ok = raise_dynamic_smem(fn, b->device, bytes) &&
+                        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block / 2, bytes) == cudaSuccess &&
+                        per_sm * b->num_sms >= b->plan.grid_ctas;
+        if (!ok) cudaGetLastError();   // a working copy too large for the device: the phased sweeps
+        return ok;
+      };
+      if (!fits(stage_off)) continue;
+      q.ok = true;
+      q.index_off = (int)idx_off;
+      q.stage_off = (int)stage_off;
+      q.smem = stage_off;
+      // The rest of a CTA's share of the shared memory for program slices (every class of CTA
+      // shape; no more than the largest program takes).
+      int optin = 0, sm = 0;
+      cudaFuncAttributes fa;
+      if (cudaFuncGetAttributes(&fa, fn) == cudaSuccess &&
+          cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device) == cudaSuccess &&
+          cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, b->device) == cudaSuccess) {
+        const int share = 1024 / block;   // CTAs per SM
+        const long long most = std::min<long long>(optin, (long long)sm / share - 1024) - (long long)fa.sharedSizeBytes - 1024;
+        long long want = 0;
+        for (ufe_mesh_h h : b->members)
+          want = std::max(want, (long long)(mode == kMixed ? h->m.max_hprog32 : h->m.max_hprog64));
+        const long long room = std::min(most - (long long)stage_off, want) / 16 * 16;
+        if (room >= 4096 && fits(stage_off + (size_t)room)) {
+          q.stage_bytes = (int)room;
+          q.smem = stage_off + (size_t)room;
+        }
       } else {
-        cudaGetLastError();   // a working copy too large for the device: the phased sweeps
+        cudaGetLastError();
       }
     }
   }
