@@ -41,7 +41,7 @@ def _nvcc() -> str:
 
 def _sources():
     return [os.path.join(SRC, f) for f in CU_SOURCES + CPP_SOURCES] + \
-        [os.path.join(SRC, "ufe_internal.h"), os.path.join(SRC, "ufe_halo.cuh"), os.path.join(HERE, "..", "include", "ufemism_gb300.h")]
+        [os.path.join(SRC, "ufe_internal.h"), os.path.join(SRC, "ufe_halo.cuh"), os.path.join(SRC, "ufe_adj_halo.cuh"), os.path.join(HERE, "..", "include", "ufemism_gb300.h")]
 
 
 def up_to_date() -> bool:

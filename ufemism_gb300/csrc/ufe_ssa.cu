@@ -33,13 +33,16 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <numeric>
+#include <thread>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -1443,21 +1446,45 @@ __global__ void k_krylov_sub(int n, const double *x, const double *mu, double *y
   if (e < n) y[e] = x[e] - mu[e];
 }
 
-// Block partial sums of V_i . w: part[i * gridDim.x + block], i = blockIdx.y.
-__global__ void k_krylov_dots(int n, const double *V, size_t ld, const double *w, double *part) {
-  const double *v = V + (size_t)blockIdx.y * ld;
-  double acc = 0.0;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) acc = fma(v[e], w[e], acc);
-  __shared__ double sw[32];
-  acc = warp_sum(acc);
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) sw[wid] = acc;
-  __syncthreads();
-  if (wid == 0) {
-    double x = lane < (int)(blockDim.x >> 5) ? sw[lane] : 0.0;
-    x = warp_sum(x);
-    if (lane == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = x;
+// Dot products of up to eight vectors with w over a block's elements: a thread's eight partial sums
+// are loaded together and go through shared memory, where a warp sums one vector (12 FP64
+// additions in a row, 64 cycles each, against 5 per vector and warp in turn). Fixed order. 16k
+// vertices, 17 vectors: 22 -> 12 us.
+constexpr int kKrylovThreads = 256, kKrylovChunk = 8;
+__device__ __forceinline__ void krylov_chunk_dots(int n, int nvec, const double *V, size_t ld, const double *w, double *out,
+                                                  double (*sacc)[kKrylovThreads]) {
+  double acc[kKrylovChunk];
+#pragma unroll
+  for (int i = 0; i < kKrylovChunk; ++i) acc[i] = 0.0;
+  for (int e = blockIdx.x * kKrylovThreads + threadIdx.x; e < n; e += gridDim.x * kKrylovThreads) {
+    const double x = w[e];
+    double v[kKrylovChunk];
+#pragma unroll
+    for (int i = 0; i < kKrylovChunk; ++i) v[i] = i < nvec ? V[(size_t)i * ld + e] : 0.0;
+#pragma unroll
+    for (int i = 0; i < kKrylovChunk; ++i)
+      if (i < nvec) acc[i] = fma(v[i], x, acc[i]);
   }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kKrylovChunk; ++i) sacc[i][threadIdx.x] = acc[i];
+  __syncthreads();
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (wid < nvec) {
+    double x = 0.0;
+#pragma unroll
+    for (int q = 0; q < kKrylovThreads / 32; ++q) x += sacc[wid][q * 32 + lane];
+    x = warp_sum(x);
+    if (lane == 0) out[(size_t)wid * gridDim.x + blockIdx.x] = x;
+  }
+}
+
+// Block partial sums of V_i . w: part[i * gridDim.x + block], vectors 8 blockIdx.y and on.
+__global__ void __launch_bounds__(kKrylovThreads) k_krylov_dots(int n, int nvec, const double *V, size_t ld, const double *w,
+                                                                double *part) {
+  __shared__ double sacc[kKrylovChunk][kKrylovThreads];
+  const int i0 = kKrylovChunk * blockIdx.y;
+  krylov_chunk_dots(n, min(kKrylovChunk, nvec - i0), V + (size_t)i0 * ld, ld, w, part + (size_t)i0 * gridDim.x, sacc);
 }
 
 // w -= sum_i h_i V_i (i < nvec)
@@ -1467,6 +1494,60 @@ __global__ void k_krylov_axpy(int n, int nvec, const double *V, size_t ld, const
   double acc = 0.0;
   for (int i = 0; i < nvec; ++i) acc = fma(h[i], V[(size_t)i * ld + e], acc);
   w[e] = w[e] - acc;
+}
+
+// The sums of a launch's block partials (fixed order), by a warp per vector; every block forms them.
+__device__ __forceinline__ void krylov_sums(int nvec, int nblocks, const double *part, double *h) {
+  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+  for (int i = wid; i < nvec; i += nw) {
+    double x = 0.0;
+    for (int b = lane; b < nblocks; b += 32) x += part[(size_t)i * nblocks + b];
+    x = warp_sum(x);
+    if (lane == 0) h[i] = x;
+  }
+  __syncthreads();
+}
+
+// One orthogonalisation pass: h = the sums of `part`, w -= sum_i h_i V_i, and the partials of the next
+// dot products, V_i . w (ndots = nvec) or w . w (ndots = 0). h goes to hout.
+__global__ void __launch_bounds__(kKrylovThreads) k_krylov_pass(int n, int nvec, const double *V, size_t ld, const double *part,
+                                                     double *w, double *hout, int ndots, double *next) {
+  extern __shared__ double sh[];   // h [nvec]
+  __shared__ double sacc[kKrylovChunk][kKrylovThreads];
+  krylov_sums(nvec, gridDim.x, part, sh);
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < nvec; i += blockDim.x) hout[i] = sh[i];
+  for (int e = blockIdx.x * kKrylovThreads + threadIdx.x; e < n; e += gridDim.x * kKrylovThreads) {
+    double acc = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < nvec; ++i) acc = fma(sh[i], V[(size_t)i * ld + e], acc);
+    w[e] = w[e] - acc;
+  }
+  if (ndots == 0) {
+    krylov_chunk_dots(n, 1, w, 0, w, next, sacc);
+    return;
+  }
+  for (int i0 = 0; i0 < ndots; i0 += kKrylovChunk)
+    krylov_chunk_dots(n, min(kKrylovChunk, ndots - i0), V + (size_t)i0 * ld, ld, w, next + (size_t)i0 * gridDim.x, sacc);
+}
+
+// v = w / |w| with |w| from its squares' partials; |w| and the sweeps' error flag go to hout.
+__global__ void __launch_bounds__(256) k_krylov_normalise(int n, int nblocks, const double *part, const double *w, double *v,
+                                                          double *hout, const unsigned int *flag) {
+  __shared__ double s;
+  krylov_sums(1, nblocks, part, &s);
+  if (threadIdx.x == 0) {   // the root and the quotient once per block (about 40 FP64 instructions)
+    const double nw = sqrt(s);
+    if (blockIdx.x == 0) {
+      hout[0] = nw;
+      hout[1] = flag && flag[0] ? (double)(int)flag[1] : 0.0;
+    }
+    s = nw > 0.0 ? 1.0 / nw : 0.0;
+  }
+  __syncthreads();
+  const double f = s;
+  if (f > 0.0)
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) v[e] = w[e] * f;
 }
 
 __global__ void k_krylov_scale(int n, const double *w, double f, double *v) {
@@ -1707,6 +1788,10 @@ __global__ void k_adj_geom(const AdjGeom a) {
     }
   }
 }
+
+}  // namespace ufe
+#include "ufe_adj_halo.cuh"
+namespace ufe {
 
 // ---------------------------------------------------------------------------------------
 // Gather / scatter / GL flux
@@ -3116,10 +3201,15 @@ struct AdjWork {
   double *kry = nullptr;
   size_t kry_vectors = 0;
   double *part = nullptr, *part_host = nullptr, *hdev = nullptr;
+  cudaEvent_t evh[2] = {nullptr, nullptr};   // a column's coefficients have arrived
+  AdjHalo halo;                              // the halo sweeps' program
 };
 
 void adj_free(AdjWork *w) {
   if (!w) return;
+  w->halo.free_all();
+  for (cudaEvent_t e : w->evh)
+    if (e) cudaEventDestroy(e);
   void *ptrs[] = {w->cT, w->kT, w->ee, w->kh, w->alpha, w->dinv, w->g, w->mu, w->c3, w->s, w->eta, w->fr,
                   w->inv_nb, w->K, w->stage, w->geom_int, w->geom_dbl, w->prog, w->ctl, w->kry, w->part, w->hdev};
   for (void *p : ptrs)
@@ -3190,6 +3280,9 @@ struct Krylov {
   double2 *zero;
   int sweeps = 0;
   int err = 0;
+  bool halo = false;  // the halo sweeps run (AdjHalo)
+  AdjHaloArgs ha;
+  size_t halo_smem = 0;
 };
 
 // One transposed sweep of mu (in place) with right-hand side g.
@@ -3204,12 +3297,84 @@ int kry_sweep(Krylov &k, const double2 *g) {
   if (!rc)
     rc = cuda_status(cudaLaunchCooperativeKernel((const void *)ssa_adjoint_sor, dim3(k.h->m.n_patch), dim3(kSsaBlock), args, 0, k.s),
                      "ssa_adjoint_sor");
-  k.sweeps += k.sweeps_per_apply;
+  return rc;
+}
+
+// The halo sweeps' argument block and the program's numbers, when the largest working copy fits.
+int halo_prepare(Krylov &k) {
+  const DevMesh &m = k.h->m;
+  const AdjHalo &d = k.a->halo;
+  AdjHaloArgs &q = k.ha;
+  const void *fn = (const void *)ssa_adjoint_halo;
+  std::memset(&q, 0, sizeof q);
+  q.s_off = d.max_local * 16;
+  q.index_off = (int)(((size_t)d.max_local * 24 + 15) / 16 * 16);
+  q.stage_off = (int)((q.index_off + (size_t)d.max_halo * 4 + 15) / 16 * 16);
+  int optin = 0, per_sm = 0;
+  cudaFuncAttributes fa;
+  int rc = cuda_status(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, k.h->device), "smem opt-in");
+  if (!rc) rc = cuda_status(cudaFuncGetAttributes(&fa, fn), "function attributes");
+  if (rc) return rc;
+  const long long room = (long long)optin - (long long)fa.sharedSizeBytes - (long long)q.stage_off - 1024;
+  if (room < 0) return UFE_OK;   // the phased sweeps
+  q.stage_bytes = (int)(room / 16 * 16);
+  k.halo_smem = (size_t)q.stage_off + (size_t)q.stage_bytes;
+  rc = cuda_status(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.halo_smem), "smem attribute");
+  if (!rc) rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kHaloBlock, k.halo_smem), "occupancy");
+  if (rc) return rc;
+  if (per_sm * k.h->num_sms < m.n_patch) return UFE_OK;
+  q.patch_slice = m.patch_slice;
+  q.hp_slice = d.hp_slice; q.hp_split = d.hp_split; q.slice_b0 = d.slice_b0; q.slice_w = d.slice_w; q.hrow_g = d.hrow_g;
+  q.hload_ptr = d.hload_ptr; q.hload_dev = d.hload_dev; q.hload_ex = d.hload_ex; q.hex_ptr = d.hex_ptr;
+  q.prog = d.prog; q.xch = d.xch; q.xch_stride = 6 * (size_t)d.n_export; q.alpha = k.a->alpha;
+  q.omega = k.aa.omega; q.flag = d.flag; q.timeout_ns = k.aa.timeout_ns;
+  rc = cuda_status(cudaMemsetAsync(d.flag, 0, 2 * sizeof(unsigned int), k.s), "adjoint flag");
+  if (rc) return rc;
+  AdjFill f;
+  f.n_slots = d.n_slices * kSlice; f.hrow_g = d.hrow_g; f.slice_b0 = d.slice_b0; f.slice_w = d.slice_w; f.prog = d.prog;
+  f.deg = m.deg; f.slice_e0 = m.slice_e0; f.cT = k.a->cT; f.kT = k.a->kT; f.ee = k.a->ee; f.kh = k.a->kh;
+  f.dinv = k.a->dinv; f.alpha = k.a->alpha; f.g = k.a->g; f.c3 = k.a->c3;
+  k_adj_fill<<<(unsigned)((f.n_slots + 127) / 128), 128, 0, k.s>>>(f);
+  rc = cuda_status(cudaGetLastError(), "k_adj_fill");
+  k.halo = rc == UFE_OK;
+  return rc;
+}
+
+// n sweeps from x (null: zero) on the halo program, right-hand side g or zero: y = from - S(x), or S(x).
+int halo_sweeps(Krylov &k, const double2 *x, bool use_g, int n_sweeps, const double2 *from, double2 *y) {
+  AdjHalo &d = k.a->halo;
+  AdjHaloArgs q = k.ha;
+  int rc = UFE_OK;
+  double2 *between = k.a->mu, *other = k.zero;   // rows between launches (never the one being read)
+  for (int done = 0; done < n_sweeps && !rc;) {
+    q.n_sweeps = std::min(kAdjSweeps, n_sweeps - done);
+    done += q.n_sweeps;
+    const bool last = done == n_sweeps;
+    if (d.tag > 0xffffff00u) {   // tags start again on cleared words
+      rc = cuda_status(cudaMemsetAsync(d.xch, 0, (size_t)kAdjSweeps * 6 * d.n_export * sizeof(unsigned long long), k.s), "adjoint exchange");
+      d.tag = 1;
+    }
+    q.tag0 = d.tag;
+    d.tag += (unsigned)q.n_sweeps;
+    q.x = x;
+    q.use_g = use_g ? 1 : 0;
+    q.from = last ? from : nullptr;
+    q.y = last ? y : between;
+    void *args[] = {(void *)&q};
+    if (!rc)
+      rc = cuda_status(cudaLaunchCooperativeKernel((const void *)ssa_adjoint_halo, dim3(k.h->m.n_patch), dim3(kHaloBlock), args,
+                                                   k.halo_smem, k.s), "ssa_adjoint_halo");
+    x = q.y;
+    std::swap(between, other);
+  }
   return rc;
 }
 
 // y = x - S(x; 0)
 int kry_apply(Krylov &k, const double *xin, double *y) {
+  if (k.halo)
+    return halo_sweeps(k, reinterpret_cast<const double2 *>(xin), false, k.sweeps_per_apply,
+                       reinterpret_cast<const double2 *>(xin), reinterpret_cast<double2 *>(y));
   const unsigned gp = (unsigned)((k.nP + 255) / 256), gn = (unsigned)((k.n + 255) / 256);
   k_krylov_load<<<gp, 256, 0, k.s>>>(k.nP, reinterpret_cast<const double2 *>(xin), k.a->alpha, k.a->mu, k.a->s);
   int rc = cuda_status(cudaGetLastError(), "k_krylov_load");
@@ -3224,15 +3389,19 @@ int kry_apply(Krylov &k, const double *xin, double *y) {
 // h[i] = V_i . wv for i < nvec (fixed-order sums: deterministic); also reads back the
 // sweep control block so that a failed wait is noticed.
 int kry_dots(Krylov &k, int nvec, const double *Vb, const double *wv, double *hout) {
-  k_krylov_dots<<<dim3(kKrylovBlocks, nvec), 256, 0, k.s>>>(k.n, Vb, k.ld, wv, k.a->part);
+  k_krylov_dots<<<dim3(kKrylovBlocks, (nvec + kKrylovChunk - 1) / kKrylovChunk), kKrylovThreads, 0, k.s>>>(k.n, nvec, Vb, k.ld, wv, k.a->part);
   int rc = cuda_status(cudaGetLastError(), "k_krylov_dots");
   if (!rc)
     rc = cuda_status(cudaMemcpyAsync(k.a->part_host, k.a->part, (size_t)nvec * kKrylovBlocks * sizeof(double),
                                      cudaMemcpyDeviceToHost, k.s), "dots D2H");
-  if (!rc) rc = cuda_status(cudaMemcpyAsync(k.a->ctl_host, k.a->ctl, sizeof(AdjCtl), cudaMemcpyDeviceToHost, k.s), "ctl D2H");
+  unsigned flag[2] = {0u, 0u};
+  if (!rc)
+    rc = k.halo ? cuda_status(cudaMemcpyAsync(flag, k.a->halo.flag, sizeof flag, cudaMemcpyDeviceToHost, k.s), "flag D2H")
+                : cuda_status(cudaMemcpyAsync(k.a->ctl_host, k.a->ctl, sizeof(AdjCtl), cudaMemcpyDeviceToHost, k.s), "ctl D2H");
   if (!rc) rc = cuda_status(cudaStreamSynchronize(k.s), "dots");
   if (rc) return rc;
-  if (k.a->ctl_host->err) k.err = k.a->ctl_host->err;
+  if (flag[0]) k.err = (int)flag[1];
+  if (!k.halo && k.a->ctl_host->err) k.err = k.a->ctl_host->err;
   for (int i = 0; i < nvec; ++i) {
     double t = 0.0;
     for (int b = 0; b < kKrylovBlocks; ++b) t += k.a->part_host[(size_t)i * kKrylovBlocks + b];
@@ -3257,14 +3426,21 @@ int kry_axpy(Krylov &k, int nvec, const double *Vb, const double *coef, double *
 int adj_gmres(Krylov &k, int m, double tol, int max_iter, double *rel, int *iters) {
   const unsigned gp = (unsigned)((k.nP + 255) / 256);
   // c = S(0; g)
-  k_krylov_load<<<gp, 256, 0, k.s>>>(k.nP, nullptr, k.a->alpha, k.a->mu, k.a->s);
-  int rc = cuda_status(cudaGetLastError(), "k_krylov_load");
-  if (!rc) rc = kry_sweep(k, k.a->g);
-  if (!rc) rc = cuda_status(cudaMemcpyAsync(k.c, k.a->mu, k.n * sizeof(double), cudaMemcpyDeviceToDevice, k.s), "copy c");
+  int rc;
+  if (k.halo) {
+    rc = halo_sweeps(k, nullptr, true, k.sweeps_per_apply, nullptr, reinterpret_cast<double2 *>(k.c));
+  } else {
+    k_krylov_load<<<gp, 256, 0, k.s>>>(k.nP, nullptr, k.a->alpha, k.a->mu, k.a->s);
+    rc = cuda_status(cudaGetLastError(), "k_krylov_load");
+    if (!rc) rc = kry_sweep(k, k.a->g);
+    if (!rc) rc = cuda_status(cudaMemcpyAsync(k.c, k.a->mu, k.n * sizeof(double), cudaMemcpyDeviceToDevice, k.s), "copy c");
+  }
+  k.sweeps += k.sweeps_per_apply;
   if (!rc) rc = cuda_status(cudaMemsetAsync(k.x, 0, k.n * sizeof(double), k.s), "memset x");
   if (rc) return rc;
   double beta0 = 0.0;
   if ((rc = kry_dots(k, 1, k.c, k.c, &beta0))) return rc;
+  if (k.err) return k.err;
   beta0 = std::sqrt(beta0);
   *iters = 0;
   *rel = 0.0;
@@ -3283,39 +3459,66 @@ int adj_gmres(Krylov &k, int m, double tol, int max_iter, double *rel, int *iter
       rc = cuda_status(cudaMemcpyAsync(V0, k.c, k.n * sizeof(double), cudaMemcpyDeviceToDevice, k.s), "copy r");
     } else {
       rc = kry_apply(k, k.x, k.w);
+      k.sweeps += k.sweeps_per_apply;
       if (!rc) {
         k_krylov_sub<<<(unsigned)((k.n + 255) / 256), 256, 0, k.s>>>(k.n, k.c, k.w, V0);
         rc = cuda_status(cudaGetLastError(), "k_krylov_sub");
       }
     }
     if (rc) return rc;
-    double beta = 0.0;
-    if ((rc = kry_dots(k, 1, V0, V0, &beta))) return rc;
-    beta = std::sqrt(beta);
+    double beta = beta0;
+    if (total > 0) {
+      if ((rc = kry_dots(k, 1, V0, V0, &beta))) return rc;
+      beta = std::sqrt(beta);
+    }
     if (beta <= tol * beta0) { res = beta / beta0; break; }
     k_krylov_scale<<<(unsigned)((k.n + 255) / 256), 256, 0, k.s>>>(k.n, V0, 1.0 / beta, V0);
     if ((rc = cuda_status(cudaGetLastError(), "k_krylov_scale"))) return rc;
     std::fill(gv.begin(), gv.end(), 0.0);
     gv[0] = beta;
     int j_end = 0;
+    // A column is queued whole (sweeps, two orthogonalisation passes, the new basis vector) and its
+    // coefficients come back behind it; the next column is queued before they are waited for, unless
+    // the last gain says that this one will converge.
+    auto enqueue = [&](int j) -> int {
+      double *hd = k.a->hdev, *hh = k.a->part_host + (size_t)(j & 1) * (2 * (size_t)kMaxKrylovRestart + 4);
+      const int nv = j + 1;
+      double *p1 = k.a->part, *p2 = p1 + (size_t)(kMaxKrylovRestart + 1) * kKrylovBlocks;
+      int e = kry_apply(k, k.V + (size_t)j * k.ld, k.w);
+      if (e) return e;
+      k_krylov_dots<<<dim3(kKrylovBlocks, (nv + kKrylovChunk - 1) / kKrylovChunk), kKrylovThreads, 0, k.s>>>(k.n, nv, k.V, k.ld, k.w, p1);
+      k_krylov_pass<<<kKrylovBlocks, kKrylovThreads, nv * sizeof(double), k.s>>>(k.n, nv, k.V, k.ld, p1, k.w, hd, nv, p2);
+      k_krylov_pass<<<kKrylovBlocks, kKrylovThreads, nv * sizeof(double), k.s>>>(k.n, nv, k.V, k.ld, p2, k.w, hd + nv, 0, p1);
+      k_krylov_normalise<<<kKrylovBlocks, 256, 0, k.s>>>(k.n, kKrylovBlocks, p1, k.w, k.V + (size_t)nv * k.ld, hd + 2 * nv,
+                                               k.halo ? k.a->halo.flag : nullptr);
+      e = cuda_status(cudaGetLastError(), "krylov column");
+      if (!e) e = cuda_status(cudaMemcpyAsync(hh, hd, (2 * (size_t)nv + 2) * sizeof(double), cudaMemcpyDeviceToHost, k.s), "column D2H");
+      if (!e && !k.halo) e = cuda_status(cudaMemcpyAsync(k.a->ctl_host, k.a->ctl, sizeof(AdjCtl), cudaMemcpyDeviceToHost, k.s), "ctl D2H");
+      if (!e) e = cuda_status(cudaEventRecord(k.a->evh[j & 1], k.s), "event");
+      return e;
+    };
+    int queued = 0;
     for (int j = 0; j < m && total < max_iter; ++j) {
-      double *Vj = k.V + (size_t)j * k.ld;
-      if ((rc = kry_apply(k, Vj, k.w))) return rc;
-      if ((rc = kry_dots(k, j + 1, k.V, k.w, hcol.data()))) return rc;
-      if ((rc = kry_axpy(k, j + 1, k.V, hcol.data(), k.w))) return rc;
-      if ((rc = kry_dots(k, j + 1, k.V, k.w, h2.data()))) return rc;
-      if ((rc = kry_axpy(k, j + 1, k.V, h2.data(), k.w))) return rc;
-      for (int i = 0; i <= j; ++i) hcol[i] += h2[i];
-      double nw = 0.0;
-      if ((rc = kry_dots(k, 1, k.w, k.w, &nw))) return rc;
-      nw = std::sqrt(nw);
+      if (queued <= j) {
+        if ((rc = enqueue(j))) return rc;
+        queued = j + 1;
+      }
+      const double last = j > 1 ? std::fabs(gv[j] / gv[j - 1]) : 1.0;
+      if (j + 1 < m && total + 1 < max_iter && std::fabs(gv[j]) / beta0 * last > 2.0 * tol) {
+        if ((rc = enqueue(j + 1))) return rc;
+        queued = j + 2;
+      }
+      if ((rc = cuda_status(cudaEventSynchronize(k.a->evh[j & 1]), "krylov column"))) return rc;
+      k.sweeps += k.sweeps_per_apply;
+      const double *hh = k.a->part_host + (size_t)(j & 1) * (2 * (size_t)kMaxKrylovRestart + 4);
+      for (int i = 0; i <= j; ++i) hcol[i] = hh[i] + hh[j + 1 + i];
+      const double nw = hh[2 * (j + 1)];
+      const int flag = (int)hh[2 * (j + 1) + 1];
+      if (flag) k.err = flag;
+      if (!k.halo && k.a->ctl_host->err) k.err = k.a->ctl_host->err;
       if (k.err) return k.err;
       for (int i = 0; i <= j; ++i) Hm(i, j) = hcol[i];
       Hm(j + 1, j) = nw;
-      if (nw > 0.0) {
-        k_krylov_scale<<<(unsigned)((k.n + 255) / 256), 256, 0, k.s>>>(k.n, k.w, 1.0 / nw, k.V + (size_t)(j + 1) * k.ld);
-        if ((rc = cuda_status(cudaGetLastError(), "k_krylov_scale"))) return rc;
-      }
       // Givens rotations: apply the previous ones to the new column, then make a new one
       for (int i = 0; i < j; ++i) {
         const double t = cs[i] * Hm(i, j) + sn[i] * Hm(i + 1, j);
@@ -3447,9 +3650,11 @@ extern "C" int ufe_ssa_vjp(ufe_mesh_h h, const ufe_params *p, const ufe_vjp_para
       rc = cuda_status(cudaMalloc(&a->kry, need * n2 * sizeof(double)), "krylov basis");
       if (!rc) a->kry_vectors = need;
     }
-    if (!rc && !a->part) rc = cuda_status(cudaMalloc(&a->part, (size_t)(kMaxKrylovRestart + 1) * kKrylovBlocks * sizeof(double)), "krylov dots");
+    if (!rc && !a->part) rc = cuda_status(cudaMalloc(&a->part, 2 * (size_t)(kMaxKrylovRestart + 1) * kKrylovBlocks * sizeof(double)), "krylov dots");
     if (!rc && !a->part_host) rc = cuda_status(cudaMallocHost(&a->part_host, (size_t)(kMaxKrylovRestart + 1) * kKrylovBlocks * sizeof(double)), "krylov dots host");
-    if (!rc && !a->hdev) rc = cuda_status(cudaMalloc(&a->hdev, (size_t)(kMaxKrylovRestart + 1) * sizeof(double)), "krylov coefficients");
+    if (!rc && !a->hdev) rc = cuda_status(cudaMalloc(&a->hdev, (2 * (size_t)kMaxKrylovRestart + 8) * sizeof(double)), "krylov coefficients");
+    for (cudaEvent_t &e : a->evh)
+      if (!rc && !e) rc = cuda_status(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
     if (!rc) {
       Krylov k;
       k.h = h; k.a = a; k.aa = aa; k.s = s; k.nP = (int)nP; k.n = (int)n2; k.ld = n2;
@@ -3457,11 +3662,21 @@ extern "C" int ufe_ssa_vjp(ufe_mesh_h h, const ufe_params *p, const ufe_vjp_para
       k.zero = reinterpret_cast<double2 *>(k.c + n2);
       k.sweeps_per_apply = vp && vp->sweeps_per_iteration > 0 ? vp->sweeps_per_iteration : 8;
       rc = cuda_status(cudaMemsetAsync(k.zero, 0, n2 * sizeof(double), s), "memset zero");
+      if (!rc && !a->halo.tried) {
+        try {
+          rc = adj_halo_create(h, a->halo);
+        } catch (const std::bad_alloc &) {   // no host memory for the program: the phased sweeps
+          a->halo.free_all();
+          a->halo.ok = false;
+        }
+      }
+      if (!rc && a->halo.ok) rc = halo_prepare(k);
       const int max_iter = vp && vp->max_sweeps > 0 ? vp->max_sweeps : 50000;
       if (!rc) rc = adj_gmres(k, restart, tol, max_iter, &k_rel, &k_iters);
       k_iters = k.sweeps;
       k_err = k.err;
       if (rc == UFE_DIVERGED) { rc = UFE_OK; k_rel = HUGE_VAL; k_err = UFE_DIVERGED; }
+      if (rc == UFE_TIMEOUT) set_error("ufe_ssa_vjp: a device-side bounded wait timed out");
     }
   }
   AdjGrad ag;
