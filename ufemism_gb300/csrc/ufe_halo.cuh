@@ -38,11 +38,17 @@ struct HaloSmem {
   unsigned long long wmax[2][32];      // each warp's maximum |res| of a sweep, by parity
   double num[kMaxDeg + 1], rcp_n[kMaxDeg + 1];   // n and 1 / n, for the boundary means
   // per slice: its block's offset in 16-byte units (bit 31: in the shared stage, else in the
-  // global program) and its width (bit 8: boundary)
+  // global program); its width (bit 8: boundary) and, from bit 16, its rows' offset in the block
+  // in 16-byte units
   uint2 tab[kMaxPatchSlices];
+  // per warp, colour 1's halo-free rows [0], its others [1] and colours 2..5 [2..5]: the first unit's
+  // tab entry, the number of units (one every nwarps, [0]: every warp that does not fetch) and the
+  // first unit, counted from the patch's first slice
+  uint4 sched[6][32];
 };
 constexpr unsigned kStaged = 1u << 31;
 
+template <bool kM>
 __device__ __forceinline__ void load_patch_halo(const SsaArgs &a, int b, HaloSmem &ps) {
   if (threadIdx.x < 8) {
     ps.lag_prev[threadIdx.x] = 0ull;
@@ -63,8 +69,33 @@ __device__ __forceinline__ void load_patch_halo(const SsaArgs &a, int b, HaloSme
     ps.rcp_n[n] = n > 0 ? 1.0 / (double)n : 0.0;
   }
   __syncthreads();
-  for (int s = ps.hps[0] + (int)threadIdx.x; s < ps.hps[7]; s += blockDim.x)
-    ps.tab[s - ps.hps[0]] = make_uint2((unsigned)a.hslice_b0[s], (unsigned)a.hslice_w[s] | (s >= ps.hps[5] ? 256u : 0u));
+  for (int s = ps.hps[0] + (int)threadIdx.x; s < ps.hps[7]; s += blockDim.x) {
+    const int w = a.hslice_w[s];
+    const bool boundary = s >= ps.hps[5];
+    const int row = kM ? slice_layout<true>(w, boundary).row : slice_layout<false>(w, boundary).row;
+    ps.tab[s - ps.hps[0]] = make_uint2((unsigned)a.hslice_b0[s], (unsigned)w | (boundary ? 256u : 0u) | (unsigned)(row / 16) << 16);
+  }
+  __syncthreads();
+}
+
+// The warps' schedules (after halo_stage). Units are dealt round robin over the whole sweep, so that
+// where slices are few a phase's warps are others than those of the phase before, which load their
+// next unit meanwhile. A phase of few slices costs its warps' chain of instructions, about 600 cycles
+// of which the index arithmetic was some 15%: with it tabulated here (and the thread count a constant
+// of the compilation) a mixed sweep takes 3.0 us instead of 3.4 at 4k vertices, 11.4 instead of 11.8
+// at 200k, an FP64 sweep 51.9 instead of 54.6 at 200k.
+__device__ __forceinline__ void halo_schedule(HaloSmem &ps, int nwarps, int nfetch, int per_slice) {
+  for (int i = threadIdx.x; i < 6 * nwarps; i += blockDim.x) {
+    const int f = i / nwarps, w = i % nwarps;
+    const int first = per_slice * ((f == 0 ? ps.hps[0] : f == 1 ? ps.hsplit : ps.hps[f - 1]) - ps.hps[0]);
+    const int end = per_slice * ((f == 0 ? ps.hsplit : ps.hps[f]) - ps.hps[0]);
+    const int stride = f == 0 ? nwarps - nfetch : nwarps;
+    int u = first + (w - first % nwarps + nwarps) % nwarps;
+    if (f == 0) u = w < stride ? first + w : end;
+    const int n = u < end ? (end - u + stride - 1) / stride : 0;
+    const uint2 t = n ? ps.tab[u / per_slice] : make_uint2(0u, 0u);
+    ps.sched[f][w] = make_uint4(t.x, t.y, (unsigned)n, (unsigned)u);
+  }
   __syncthreads();
 }
 
@@ -75,7 +106,7 @@ __device__ __forceinline__ void load_patch_halo(const SsaArgs &a, int b, HaloSme
 // first round's are issued before the barrier), and whole colours of at most one round, as many
 // as fit. Thread 0 plans, then the CTA copies the blocks; halo_refresh fills in the row data.
 // Warps that fetch the halo slots (the others run colour 1's halo-free rows meanwhile).
-__device__ __forceinline__ int fetch_warps(int nwarps) { return nwarps >= 16 ? 4 : nwarps >= 8 ? 2 : 1; }
+__host__ __device__ constexpr int fetch_warps(int nwarps) { return nwarps >= 16 ? 4 : nwarps >= 8 ? 2 : 1; }
 
 template <bool kM>
 __device__ void halo_stage(const SsaArgs &a, HaloSmem &ps, unsigned char *stage, int skip_tail) {
@@ -231,10 +262,10 @@ __device__ __forceinline__ void halo_poll(const SsaArgs &a, const HaloSmem &ps, 
 // What a slice's update needs besides its program, in registers across the sweep.
 struct SliceCtx {
   const HaloSmem *ps;
-  const unsigned char *stage;
-  unsigned long long *xout;    // this sweep's exchange buffer, at the patch's first export
-  unsigned tag;                // this sweep's tag
-  int base, n_own;
+  const unsigned char *stage, *prog;   // the staged and the global slices (mixed: at the lane's 16 bytes)
+  unsigned long long *xout;            // this sweep's exchange buffer, at the patch's first export
+  unsigned tag;                        // this sweep's tag
+  int n_own;
 };
 
 __device__ __forceinline__ bool is_dirichlet(const SsaArgs &a, const HaloSmem &ps, int l) {
@@ -259,22 +290,23 @@ template <> struct Prog<kMixed> {
   uint2 row;
   uint2 t;
 
-  __device__ __forceinline__ void read(const unsigned char *b, int lane) {
+  // b: the block, offset by the lane's 16 bytes
+  __device__ __forceinline__ void read(const unsigned char *b) {
     const int w = (int)(t.y & 255u);
-    const SliceLayout q = slice_layout<true>(w, false);
-    c = reinterpret_cast<const uint4 *>(b)[lane];
-    const float4 *kp = reinterpret_cast<const float4 *>(b + q.coef) + lane;
+    c = *reinterpret_cast<const uint4 *>(b);
+    const unsigned char *kp = b + 512;   // the coefficients of slices of up to eight entries
+    if (w > 8) kp = b + slice_layout<true>(w, false).coef;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) k[i] = kp[i * kSlice];
-    if (w > 6) k[3] = kp[3 * kSlice];
-    row = reinterpret_cast<const uint2 *>(b + q.row)[lane];
-    sd = reinterpret_cast<const float4 *>(b + q.dat)[lane];
+    for (int i = 0; i < 3; ++i) k[i] = *reinterpret_cast<const float4 *>(kp + 512 * i);
+    if (w > 6) k[3] = *reinterpret_cast<const float4 *>(kp + 3 * 512);
+    const unsigned char *r = b + (t.y >> 16) * 16u;
+    row = *reinterpret_cast<const uint2 *>(r - (threadIdx.x & 31) * 8);
+    sd = *reinterpret_cast<const float4 *>(r + 256);
   }
-  __device__ __forceinline__ void load(const SsaArgs &a, const SliceCtx &x, int unit) {
-    t = x.ps->tab[unit - x.base];
-    const int lane = threadIdx.x & 31;
-    if (t.x & kStaged) read(x.stage + 16 * (size_t)(t.x & ~kStaged), lane);
-    else read(a.hprog + 16 * (size_t)t.x, lane);
+  __device__ __forceinline__ void load(const SliceCtx &x, uint2 entry, int) {
+    t = entry;
+    if (t.x & kStaged) read(x.stage + 16u * (t.x & ~kStaged));
+    else read(x.prog + 16 * (size_t)t.x);
   }
   __device__ __forceinline__ void update(const SsaArgs &a, const SliceCtx &x, int, float2 *ld, float omega, float &mx) const {
     const unsigned l = row.x & 0xffffu, ex = row.x >> 16;
@@ -297,12 +329,11 @@ template <> struct Prog<kMixed> {
       entry(6);
       entry(7);
       if (w > 8) {   // the entries beyond the eighth, from the block
-        const unsigned char *b = (t.x & kStaged) ? x.stage + 16 * (size_t)(t.x & ~kStaged) : a.hprog + 16 * (size_t)t.x;
-        const int lane = threadIdx.x & 31;
+        const unsigned char *b = (t.x & kStaged) ? x.stage + 16u * (t.x & ~kStaged) : x.prog + 16 * (size_t)t.x;
         const SliceLayout y = slice_layout<true>(w, false);
         for (int q = 8; q < w; ++q) {
-          const float2 cc = reinterpret_cast<const float2 *>(b + y.coef + (q / 2) * 512 + lane * 16)[q % 2];
-          const float2 v = ld[reinterpret_cast<const uint16_t *>(b + (q / 8) * 512 + lane * 16)[q % 8]];
+          const float2 cc = reinterpret_cast<const float2 *>(b + y.coef + (q / 2) * 512)[q % 2];
+          const float2 v = ld[reinterpret_cast<const uint16_t *>(b + (q / 8) * 512)[q % 8]];
           su = fmaf(v.x, cc.x, su);
           sv = fmaf(v.y, cc.y, sv);
         }
@@ -336,24 +367,24 @@ template <int kMode> struct Prog {
   __device__ __forceinline__ void read(const unsigned char *p, int unit) {
     const int w = (int)(t.y & 255u), lane = threadIdx.x & 31;
     const int rl = (unit & 1) * 16 + (lane & 15), rc = 2 * rl + (lane >> 4);
-    const SliceLayout q = slice_layout<false>(w, false);
     c = reinterpret_cast<const uint4 *>(p)[rl];
-    const double *kp = reinterpret_cast<const double *>(p + q.coef) + rc;
+    const double *kp = reinterpret_cast<const double *>(p + (w > 8 ? slice_layout<false>(w, false).coef : 512)) + rc;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       if (i < w) k[i] = kp[i * 2 * kSlice];
-    const uint4 rw = reinterpret_cast<const uint4 *>(p + q.row)[rl];
+    const unsigned char *r0 = p + (t.y >> 16) * 16u;
+    const uint4 rw = reinterpret_cast<const uint4 *>(r0)[rl];
     row = rw.x;
     s3 = __hiloint2double((int)rw.w, (int)rw.z);
-    const double *d = reinterpret_cast<const double *>(p + q.dat) + rc;
+    const double *d = reinterpret_cast<const double *>(r0 + 512) + rc;
     r = d[0];
     b = d[2 * kSlice];
     if (kExact) rcp = d[4 * kSlice];
   }
-  __device__ __forceinline__ void load(const SsaArgs &a, const SliceCtx &x, int unit) {
-    t = x.ps->tab[(unit >> 1) - x.base];
-    if (t.x & kStaged) read(x.stage + 16 * (size_t)(t.x & ~kStaged), unit);
-    else read(a.hprog + 16 * (size_t)t.x, unit);
+  __device__ __forceinline__ void load(const SliceCtx &x, uint2 entry, int unit) {
+    t = entry;
+    if (t.x & kStaged) read(x.stage + 16u * (t.x & ~kStaged), unit);
+    else read(x.prog + 16 * (size_t)t.x, unit);
   }
   __device__ __forceinline__ static void add(double u, double cc, double &s) {
     if (kExact) s = s + u * cc;
@@ -370,7 +401,7 @@ template <int kMode> struct Prog {
       ui = ld[2 * l];
       const double uo = ld[2 * (int)l + 1 - 2 * comp];   // the row's other component
       un = ui;
-      if ((int)l < x.n_own) reinterpret_cast<double *>(a.hundo)[32 * unit + 2 * (lane & 15) + comp] = ui;
+      if ((int)l < x.n_own) reinterpret_cast<double *>(a.hundo)[(size_t)64 * x.ps->hps[0] + 32 * unit + 2 * (lane & 15) + comp] = ui;
       if (a.skip && is_dirichlet(a, *x.ps, (int)l)) {
         put = false;
       } else {
@@ -382,7 +413,7 @@ template <int kMode> struct Prog {
             if (j != kNoCol) add(ld[2 * j], k[q], su);
           }
         if (w > 8) {
-          const unsigned char *p = (t.x & kStaged) ? x.stage + 16 * (size_t)(t.x & ~kStaged) : a.hprog + 16 * (size_t)t.x;
+          const unsigned char *p = (t.x & kStaged) ? x.stage + 16u * (t.x & ~kStaged) : x.prog + 16 * (size_t)t.x;
           const SliceLayout y = slice_layout<false>(w, false);
           const int rl = (unit & 1) * 16 + (lane & 15);
           for (int q = 8; q < w; ++q) {
@@ -419,17 +450,17 @@ template <int kMode> struct Prog {
 // updated in phase 5), as phase_boundary. Mixed: c0 + mean of the corrections (phase_boundary).
 // FP64: a lane a component, as in the colour phases.
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ const unsigned char *slice_block(const SsaArgs &a, const SliceCtx &x, uint2 t) {
-  return (t.x & kStaged) ? x.stage + 16 * (size_t)(t.x & ~kStaged) : a.hprog + 16 * (size_t)t.x;
+__device__ __forceinline__ const unsigned char *slice_block(const SliceCtx &x, uint2 t) {
+  return (t.x & kStaged) ? x.stage + 16u * (t.x & ~kStaged) : x.prog + 16 * (size_t)t.x;
 }
 
 __device__ void halo_boundary(const SsaArgs &a, const SliceCtx &x, int s_begin, int s_end, int nwarps, float2 *ld) {
   const int lane = threadIdx.x & 31;
   for (int s = s_begin + (int)(threadIdx.x >> 5); s < s_end; s += nwarps) {
-    const uint2 t = x.ps->tab[s - x.base];
+    const uint2 t = x.ps->tab[s - x.ps->hps[0]];
     const int w = (int)(t.y & 255u);
     const SliceLayout y = slice_layout<true>(w, true);
-    const unsigned char *b = slice_block(a, x, t);
+    const unsigned char *b = slice_block(x, t) - 16 * lane;
     const uint4 c = reinterpret_cast<const uint4 *>(b)[lane];
     const unsigned rw = reinterpret_cast<const uint2 *>(b + y.row)[lane].x;
     const float4 c0 = reinterpret_cast<const float4 *>(b + y.dat)[lane];
@@ -462,10 +493,10 @@ __device__ void halo_boundary(const SsaArgs &a, const SliceCtx &x, int s_begin, 
   const int lane = threadIdx.x & 31, comp = lane >> 4;
   double *const ld = reinterpret_cast<double *>(ld2) + comp;
   for (int unit = 2 * s_begin + (int)(threadIdx.x >> 5); unit < 2 * s_end; unit += nwarps) {
-    const uint2 t = x.ps->tab[(unit >> 1) - x.base];
+    const uint2 t = x.ps->tab[(unit >> 1) - x.ps->hps[0]];
     const int w = (int)(t.y & 255u), rl = (unit & 1) * 16 + (lane & 15);
     const SliceLayout y = slice_layout<false>(w, true);
-    const unsigned char *b = slice_block(a, x, t);
+    const unsigned char *b = slice_block(x, t);
     const uint4 c = reinterpret_cast<const uint4 *>(b)[rl];
     const unsigned rw = reinterpret_cast<const uint4 *>(b + y.row)[rl].x;
     const unsigned l = rw & 0xffffu, ex = rw >> 16;
@@ -607,27 +638,39 @@ __device__ __forceinline__ int halo_decide(const SsaArgs &a, const Team &t, Halo
 // The whole solve_SSA of one problem on the halo sweeps, run by the CTAs of a team (each CTA owns
 // one patch). Returns false when a bounded wait failed; the error is recorded in the problem's
 // control block and the team's barrier counter.
-template <int kMode, class Team>
+template <int kMode, int kThreads, class Team>
 __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
   constexpr bool kM = kMode == kMixed;
   using T = typename std::conditional<kM, float2, double2>::type;
   using Mx = typename std::conditional<kM, float, unsigned long long>::type;
   using Om = typename std::conditional<kM, float, double>::type;
+  constexpr int nwarps = kThreads / 32;
   SsaCtl *ctl = a.ctl;
   const bool leader = t.rank() == 0 && threadIdx.x == 0;
   __shared__ HaloSmem ps;
   extern __shared__ __align__(16) unsigned char ufe_local_rows[];
   __syncthreads();   // batched members: every thread is done with the last member's patch
-  load_patch_halo(a, t.rank(), ps);
+  load_patch_halo<kM>(a, t.rank(), ps);
   T *const ld = reinterpret_cast<T *>(ufe_local_rows);
   int *const hidx = reinterpret_cast<int *>(ufe_local_rows + (size_t)a.halo_index_off);
   unsigned char *const stage = ufe_local_rows + (size_t)a.stage_off;
   for (int i = threadIdx.x; i < ps.nh; i += blockDim.x) hidx[i] = a.hload_ex[ps.hl0 + i];
   halo_stage<kM>(a, ps, stage, kMode == kFast64 ? 512 : 0);
-  const int wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;   // nwarps: a power of two
-  const int nfetch = fetch_warps(nwarps);
+  constexpr int kU = Prog<kMode>::kPerSlice;
+  halo_schedule(ps, nwarps, fetch_warps(nwarps), kU);
+  const int wid = threadIdx.x >> 5;
+  constexpr int nfetch = fetch_warps(nwarps);
   const int decider = (int)blockDim.x - nfetch * kSlice;        // first thread of the fetch warps
-  const int base = ps.hps[0], split = ps.hsplit, n_own = ps.n_own, ex_first = ps.ex0 * (kM ? 2 : 4);
+  const int n_own = ps.n_own;
+  const bool any_edges = ps.hps[6] > ps.hps[5], any_corners = ps.hps[7] > ps.hps[6];
+  SliceCtx x{&ps, stage, a.hprog, a.hxch + (size_t)ps.ex0 * (kM ? 2 : 4), 0u, n_own};
+  if (kM) {
+    x.stage += 16 * (threadIdx.x & 31);
+    x.prog += 16 * (threadIdx.x & 31);
+  }
+  // the exchange buffers in turn: xout is the next sweep's, xin (for the readers) the last one's
+  const unsigned long long *xin = a.hxch;
+  int turn = 0;
   const T zero{0, 0};
   // The own rows of the working copy: corrections (mixed) start from zero, velocities from UV.
   for (int i = threadIdx.x; i < ps.n_own; i += blockDim.x) {
@@ -678,6 +721,7 @@ __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
     int sweeps = 0;
     bool lin_done = false, synced = true;   // synced: a barrier follows the previous sweep, which is decided
     int did_reset = 0;
+    int until_refold = a.refold;            // (refold > 0)
     unsigned last_G = 0;                    // the sweep that decided (or ended) the linear solve
     halo_refresh<kMode>(a, ps, stage);
     UFE_TM(kTmOther);
@@ -685,21 +729,28 @@ __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
       ++sweeps;
       UFE_TM_COUNT(kTmSweeps);
       const unsigned G = gsweep++;
-      const SliceCtx x{&ps, stage, a.hxch + (size_t)(G % kXchBufs) * a.xch_stride + (size_t)ex_first, G + 1u, base, n_own};
+      x.tag = G + 1u;
       Mx mx = 0;
       Prog<kMode> pr;
-      constexpr int kU = Prog<kMode>::kPerSlice;
-      // Units are dealt round robin over the whole sweep, so that a phase's warps are others than
-      // those of the phase before where slices are few; each phase's first unit is loaded before
-      // the barrier that the phase waits for.
-      auto first_unit = [&](int s_begin) { return kU * s_begin + ((wid - kU * (s_begin - base)) & (nwarps - 1)); };
+      // a phase's units of this warp (the first is loaded)
+      uint4 sc = make_uint4(0u, 0u, 0u, 0u);
+      auto run = [&](int stride) {
+        while (sc.z) {
+          pr.update(a, x, (int)sc.w, ld, omega, mx);
+          if (--sc.z == 0u) break;
+          sc.w += (unsigned)stride;
+          pr.load(x, ps.tab[sc.w / kU], (int)sc.w);
+        }
+      };
+      auto next = [&](int f) {   // the phase's first unit, loaded before the barrier that the phase waits for
+        sc = ps.sched[f][wid];
+        if (sc.z) pr.load(x, make_uint2(sc.x, sc.y), (int)sc.w);
+      };
       // colour 1's halo-free rows; meanwhile the last warps fetch the halo slots and their first
       // thread the decision on the sweep before
       if (wid < nwarps - nfetch) {
-        for (int u = kU * base + wid; u < kU * split; u += nwarps - nfetch) {
-          pr.load(a, x, u);
-          pr.update(a, x, u, ld, omega, mx);
-        }
+        next(0);
+        run(nwarps - nfetch);
       } else if (synced) {
         for (int i = (int)threadIdx.x - decider; i < ps.nh; i += nfetch * kSlice) {
           if constexpr (kM) ld[n_own + i] = zero;
@@ -709,24 +760,17 @@ __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
       } else {
         unsigned long long word = 0ull;
         if ((int)threadIdx.x == decider) word = halo_word(a, G - 1u);   // in flight with the halo slots
-        halo_poll(a, ps, a.hxch + (size_t)((G + kXchBufs - 1u) % kXchBufs) * a.xch_stride, G, t.bar(), hidx, ld, nfetch);
+        halo_poll(a, ps, xin, G, t.bar(), hidx, ld, nfetch);
         if ((int)threadIdx.x == decider) ps.act[G & 1] = halo_decide(a, t, ps, G - 1u, word);
       }
-      int u = first_unit(split);
-      if (u < kU * ps.hps[1]) pr.load(a, x, u);
+      next(1);
       __syncthreads();
       UFE_TM(kTmWaitColour);
 #pragma unroll 1
-      for (int f = 0; f < 5; ++f) {
-        const int s_end = ps.hps[f + 1];
-        while (u < kU * s_end) {
-          pr.update(a, x, u, ld, omega, mx);
-          u += nwarps;
-          if (u < kU * s_end) pr.load(a, x, u);
-        }
-        if (f < 4) {
-          u = first_unit(s_end);
-          if (u < kU * ps.hps[f + 2]) pr.load(a, x, u);
+      for (int f = 1; f < 6; ++f) {
+        run(nwarps);
+        if (f < 5) {
+          next(f + 1);
         } else {
           if constexpr (kM) {
             const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
@@ -737,21 +781,28 @@ __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
           }
         }
         __syncthreads();
-        UFE_TM_SUB(kTmColour0 + f);
+        UFE_TM_SUB(kTmColour0 + f - 1);
       }
       UFE_TM(kTmColour);
       if (wid == 0) halo_arrive<kM>(a, t, ps, G);
       UFE_TM(kTmArrive);
-#pragma unroll 1
-      for (int f = 5; f < 7; ++f) {
-        if (ps.hps[f + 1] == ps.hps[f]) continue;
-        halo_boundary(a, x, ps.hps[f], ps.hps[f + 1], nwarps, ld);
+      if (any_edges) {
+        halo_boundary(a, x, ps.hps[5], ps.hps[6], nwarps, ld);
         __syncthreads();
       }
+      if (any_corners) {
+        halo_boundary(a, x, ps.hps[6], ps.hps[7], nwarps, ld);
+        __syncthreads();
+      }
+      // the exchange buffers move on
+      xin = a.hxch + (size_t)turn * a.xch_stride;
+      turn = turn == kXchBufs - 1 ? 0 : turn + 1;
+      x.xout = a.hxch + (size_t)turn * a.xch_stride + (size_t)ps.ex0 * (kM ? 2 : 4);
       UFE_TM(kTmBoundary);
       int act = ps.act[G & 1];
       if (act < 0) return false;
-      const bool refold_now = kM && a.refold > 0 && sweeps % a.refold == 0;
+      const bool refold_now = kM && --until_refold == 0;
+      if (refold_now) until_refold = a.refold;
       synced = false;
       last_G = G;
       if (act != 0) {

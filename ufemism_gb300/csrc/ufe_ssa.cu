@@ -164,8 +164,8 @@ constexpr size_t kLocalRowsMaxBytes = 160 * 1024;
 constexpr int kMaxKrylovRestart = 1000;   // largest GMRES restart length of the VJP
 // Threads per CTA of the halo sweeps: 128 registers hold a slice's program across a barrier. On
 // the 200k dome a mixed sweep measured 18.1 us with 1024 threads (64 registers, spilled), 13.7 with
-// 512 and 18.0 with 256; at 16k vertices 8.6, 5.1 and 5.0 (before the row updates were shortened,
-// which left 12.1 and 4.3 at 512).
+// 512 and 18.0 with 256; at 16k vertices 8.6, 5.1 and 5.0 (since then the row updates were shortened
+// and the warps' schedules tabulated, which left 11.4 and 3.4 at 512).
 constexpr int kHaloBlock = 512;
 
 // Per-phase timers of the persistent solver (profiling build only, -DUFE_PHASE_TIMERS=1):
@@ -1219,7 +1219,7 @@ template <int kMode, bool kHalo>
 __global__ void __launch_bounds__(kHalo ? kHaloBlock : kSsaBlock, kCtasPerSm)
     ssa_persistent(const __grid_constant__ SsaArgs a) {
   GridTeam t{&a.ctl->bar_count, 0u};
-  if constexpr (kHalo) solve_member_halo<kMode>(a, t);
+  if constexpr (kHalo) solve_member_halo<kMode, kHaloBlock>(a, t);
   else solve_member<kMode>(a, t);
 }
 
@@ -1261,7 +1261,7 @@ __global__ void __launch_bounds__(kBlock, kPerSm) ssa_batched(const BatchArgs b)
     if (m >= (unsigned)b.n_members) return;
     stage_args(a, b.members + m);
     bool ok;
-    if constexpr (kHalo) ok = solve_member_halo<kMode>(a, t);
+    if constexpr (kHalo) ok = solve_member_halo<kMode, kBlock>(a, t);
     else ok = solve_member<kMode>(a, t);
     if (!ok) {
       if (threadIdx.x == 0) atomicCAS(b.err, 0, (int)UFE_TIMEOUT);
