@@ -41,10 +41,10 @@ struct HaloSmem {
   // global program); its width (bit 8: boundary) and, from bit 16, its rows' offset in the block
   // in 16-byte units
   uint2 tab[kMaxPatchSlices];
-  // per warp, colour 1's halo-free rows [0], its others [1] and colours 2..5 [2..5]: the first unit's
-  // tab entry, the number of units (one every nwarps, [0]: every warp that does not fetch) and the
-  // first unit, counted from the patch's first slice
-  uint4 sched[6][32];
+  // per warp, colour 1's halo-free rows [0], its others [1], colours 2..5 [2..5] and the boundary
+  // rows [6]: the first unit's tab entry, the number of units (one every nwarps, [0]: every warp that
+  // does not fetch) and the first unit, counted from the patch's first slice
+  uint4 sched[7][32];
 };
 constexpr unsigned kStaged = 1u << 31;
 
@@ -85,10 +85,10 @@ __device__ __forceinline__ void load_patch_halo(const SsaArgs &a, int b, HaloSme
 // of the compilation) a mixed sweep takes 3.0 us instead of 3.4 at 4k vertices, 11.4 instead of 11.8
 // at 200k, an FP64 sweep 51.9 instead of 54.6 at 200k.
 __device__ __forceinline__ void halo_schedule(HaloSmem &ps, int nwarps, int nfetch, int per_slice) {
-  for (int i = threadIdx.x; i < 6 * nwarps; i += blockDim.x) {
+  for (int i = threadIdx.x; i < 7 * nwarps; i += blockDim.x) {
     const int f = i / nwarps, w = i % nwarps;
     const int first = per_slice * ((f == 0 ? ps.hps[0] : f == 1 ? ps.hsplit : ps.hps[f - 1]) - ps.hps[0]);
-    const int end = per_slice * ((f == 0 ? ps.hsplit : ps.hps[f]) - ps.hps[0]);
+    const int end = per_slice * ((f == 0 ? ps.hsplit : f == 6 ? ps.hps[7] : ps.hps[f]) - ps.hps[0]);
     const int stride = f == 0 ? nwarps - nfetch : nwarps;
     int u = first + (w - first % nwarps + nwarps) % nwarps;
     if (f == 0) u = w < stride ? first + w : end;
@@ -448,59 +448,82 @@ template <int kMode> struct Prog {
 // Boundary phase f (5: edge rows, 6: corners) of apply_Neumann_boundary_AaAc: the mean of the
 // listed neighbours (edge rows: the non-edge ones; corners: all, the edge rows among them already
 // updated in phase 5), as phase_boundary. Mixed: c0 + mean of the corrections (phase_boundary).
-// FP64: a lane a component, as in the colour phases.
+// FP64: a lane a component, as in the colour phases. The patches with edges and corners run two more
+// phases than the others, which wait for them: their first slice's program is loaded before the
+// barrier that ends colour 5, by warps dealt as in the colour phases, and the arrival is another
+// warp's. The four corner patches' part of a mixed sweep went from 1400 to 920 cycles (4k vertices).
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ const unsigned char *slice_block(const SliceCtx &x, uint2 t) {
-  return (t.x & kStaged) ? x.stage + 16u * (t.x & ~kStaged) : x.prog + 16 * (size_t)t.x;
-}
+template <int kMode> struct BoundaryProg;
 
-__device__ void halo_boundary(const SsaArgs &a, const SliceCtx &x, int s_begin, int s_end, int nwarps, float2 *ld) {
-  const int lane = threadIdx.x & 31;
-  for (int s = s_begin + (int)(threadIdx.x >> 5); s < s_end; s += nwarps) {
-    const uint2 t = x.ps->tab[s - x.ps->hps[0]];
+template <> struct BoundaryProg<kMixed> {
+  uint4 c;
+  float4 c0;      // (c0 x, c0 y, 1 / count, -)
+  uint2 t;
+  unsigned row;
+
+  __device__ __forceinline__ static const unsigned char *block(const SliceCtx &x, uint2 t) {
+    return (t.x & kStaged) ? x.stage + 16u * (t.x & ~kStaged) : x.prog + 16 * (size_t)t.x;
+  }
+  __device__ __forceinline__ void load(const SliceCtx &x, uint2 entry, int) {
+    t = entry;
+    const unsigned char *b = block(x, t), *r = b + (t.y >> 16) * 16u;
+    c = *reinterpret_cast<const uint4 *>(b);
+    row = *reinterpret_cast<const unsigned *>(r - (threadIdx.x & 31) * 8);
+    c0 = *reinterpret_cast<const float4 *>(r + 256);
+  }
+  __device__ __forceinline__ void update(const SsaArgs &, const SliceCtx &x, int, float2 *ld) const {
+    const unsigned l = row & 0xffffu, ex = row >> 16;
+    if (l == kNoCol) return;
     const int w = (int)(t.y & 255u);
-    const SliceLayout y = slice_layout<true>(w, true);
-    const unsigned char *b = slice_block(x, t) - 16 * lane;
-    const uint4 c = reinterpret_cast<const uint4 *>(b)[lane];
-    const unsigned rw = reinterpret_cast<const uint2 *>(b + y.row)[lane].x;
-    const float4 c0 = reinterpret_cast<const float4 *>(b + y.dat)[lane];
-    const unsigned l = rw & 0xffffu, ex = rw >> 16;
-    if (l == kNoCol) continue;
     float sx = 0.0f, sy = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    auto entry = [&](int q) {   // (a row's entries come first)
       const unsigned j = packed_col(c, q);
       if (j != kNoCol) {
         const float2 u = ld[j];
         sx = sx + u.x;
         sy = sy + u.y;
       }
-    }
-    for (int q = 8; q < w; ++q) {
-      const unsigned j = reinterpret_cast<const uint16_t *>(b + (q / 8) * 512 + lane * 16)[q % 8];
-      if (j == kNoCol) break;
-      const float2 u = ld[j];
-      sx = sx + u.x;
-      sy = sy + u.y;
+    };
+#pragma unroll
+    for (int q = 0; q < 4; ++q) entry(q);
+    if (w > 4) {
+#pragma unroll
+      for (int q = 4; q < 8; ++q) entry(q);
+      const unsigned char *b = block(x, t);
+      for (int q = 8; q < w; ++q) {
+        const unsigned j = reinterpret_cast<const uint16_t *>(b + (q / 8) * 512)[q % 8];
+        if (j == kNoCol) break;
+        const float2 u = ld[j];
+        sx = sx + u.x;
+        sy = sy + u.y;
+      }
     }
     const float2 nv = make_float2(fmaf(sx, c0.z, c0.x), fmaf(sy, c0.z, c0.y));
     ld[l] = nv;
     if (ex != kNoCol) export_value(x.xout + 2 * ex, x.tag, nv);
   }
-}
+};
 
-__device__ void halo_boundary(const SsaArgs &a, const SliceCtx &x, int s_begin, int s_end, int nwarps, double2 *ld2) {
-  const int lane = threadIdx.x & 31, comp = lane >> 4;
-  double *const ld = reinterpret_cast<double *>(ld2) + comp;
-  for (int unit = 2 * s_begin + (int)(threadIdx.x >> 5); unit < 2 * s_end; unit += nwarps) {
-    const uint2 t = x.ps->tab[(unit >> 1) - x.ps->hps[0]];
-    const int w = (int)(t.y & 255u), rl = (unit & 1) * 16 + (lane & 15);
-    const SliceLayout y = slice_layout<false>(w, true);
-    const unsigned char *b = slice_block(x, t);
-    const uint4 c = reinterpret_cast<const uint4 *>(b)[rl];
-    const unsigned rw = reinterpret_cast<const uint4 *>(b + y.row)[rl].x;
-    const unsigned l = rw & 0xffffu, ex = rw >> 16;
-    if (l == kNoCol) continue;
+template <int kMode> struct BoundaryProg {
+  uint4 c;
+  uint2 t;
+  unsigned row;
+
+  __device__ __forceinline__ static const unsigned char *block(const SliceCtx &x, uint2 t) {
+    return (t.x & kStaged) ? x.stage + 16u * (t.x & ~kStaged) : x.prog + 16 * (size_t)t.x;
+  }
+  __device__ __forceinline__ void load(const SliceCtx &x, uint2 entry, int unit) {
+    t = entry;
+    const int rl = (unit & 1) * 16 + (threadIdx.x & 15);
+    const unsigned char *b = block(x, t);
+    c = reinterpret_cast<const uint4 *>(b)[rl];
+    row = reinterpret_cast<const uint4 *>(b + (t.y >> 16) * 16u)[rl].x;
+  }
+  __device__ __forceinline__ void update(const SsaArgs &a, const SliceCtx &x, int unit, double2 *ld2) const {
+    const unsigned l = row & 0xffffu, ex = row >> 16;
+    if (l == kNoCol) return;
+    const int lane = threadIdx.x & 31, comp = lane >> 4, w = (int)(t.y & 255u), rl = (unit & 1) * 16 + (lane & 15);
+    double *const ld = reinterpret_cast<double *>(ld2) + comp;
     double s = 0.0;
     int nvals = 0;
 #pragma unroll
@@ -511,19 +534,22 @@ __device__ void halo_boundary(const SsaArgs &a, const SliceCtx &x, int s_begin, 
         ++nvals;
       }
     }
-    for (int q = 8; q < w; ++q) {
-      const unsigned j = reinterpret_cast<const uint16_t *>(b + (q / 8) * 512 + rl * 16)[q % 8];
-      if (j == kNoCol) break;
-      s = s + ld[2 * j];
-      ++nvals;
+    if (w > 8) {
+      const unsigned char *b = block(x, t);
+      for (int q = 8; q < w; ++q) {
+        const unsigned j = reinterpret_cast<const uint16_t *>(b + (q / 8) * 512 + rl * 16)[q % 8];
+        if (j == kNoCol) break;
+        s = s + ld[2 * j];
+        ++nvals;
+      }
     }
     if (nvals < a.ncm) s = s + 0.0;
     const double nv = divide_by(s, x.ps->num[nvals], x.ps->rcp_n[nvals]);
-    if ((int)l < x.n_own) reinterpret_cast<double *>(a.hundo)[32 * unit + 2 * (lane & 15) + comp] = ld[2 * l];
+    if ((int)l < x.n_own) reinterpret_cast<double *>(a.hundo)[(size_t)64 * x.ps->hps[0] + 32 * unit + 2 * (lane & 15) + comp] = ld[2 * l];
     ld[2 * l] = nv;
     if (ex != kNoCol) export_value(x.xout + 4 * ex + 2 * comp, x.tag, nv);
   }
-}
+};
 
 // Per-slot copies of the row data a sweep reads that change between linear solves (mixed: the
 // FP32 reciprocals of the centre coefficients and the defect; fast FP64: the reciprocals and the
@@ -662,14 +688,15 @@ __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
   constexpr int nfetch = fetch_warps(nwarps);
   const int decider = (int)blockDim.x - nfetch * kSlice;        // first thread of the fetch warps
   const int n_own = ps.n_own;
-  const bool any_edges = ps.hps[6] > ps.hps[5], any_corners = ps.hps[7] > ps.hps[6];
-  SliceCtx x{&ps, stage, a.hprog, a.hxch + (size_t)ps.ex0 * (kM ? 2 : 4), 0u, n_own};
+  const bool any_boundary = ps.hps[7] > ps.hps[5], any_corners = ps.hps[7] > ps.hps[6];
+  const int ex_first = ps.ex0 * (kM ? 2 : 4);
+  SliceCtx x{&ps, stage, a.hprog, a.hxch + ex_first, 0u, n_own};
   if (kM) {
     x.stage += 16 * (threadIdx.x & 31);
     x.prog += 16 * (threadIdx.x & 31);
   }
   // the exchange buffers in turn: xout is the next sweep's, xin (for the readers) the last one's
-  const unsigned long long *xin = a.hxch;
+  unsigned long long *xin = a.hxch;
   int turn = 0;
   const T zero{0, 0};
   // The own rows of the working copy: corrections (mixed) start from zero, velocities from UV.
@@ -767,44 +794,58 @@ __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
       __syncthreads();
       UFE_TM(kTmWaitColour);
 #pragma unroll 1
-      for (int f = 1; f < 6; ++f) {
+      for (int f = 1;; ++f) {
         run(nwarps);
-        if (f < 5) {
-          next(f + 1);
-        } else {
-          if constexpr (kM) {
-            const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-            if ((threadIdx.x & 31) == 0) ps.wmax[G & 1][wid] = m;
-          } else {
-            const unsigned long long m = warp_max_u64(mx);
-            if ((threadIdx.x & 31) == 0) ps.wmax[G & 1][wid] = m;
-          }
-        }
+        if (f == 5) break;
+        next(f + 1);
         __syncthreads();
         UFE_TM_SUB(kTmColour0 + f - 1);
       }
-      UFE_TM(kTmColour);
-      if (wid == 0) halo_arrive<kM>(a, t, ps, G);
-      UFE_TM(kTmArrive);
-      if (any_edges) {
-        halo_boundary(a, x, ps.hps[5], ps.hps[6], nwarps, ld);
-        __syncthreads();
+      if constexpr (kM) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+        if ((threadIdx.x & 31) == 0) ps.wmax[G & 1][wid] = m;
+      } else {
+        const unsigned long long m = warp_max_u64(mx);
+        if ((threadIdx.x & 31) == 0) ps.wmax[G & 1][wid] = m;
       }
-      if (any_corners) {
-        halo_boundary(a, x, ps.hps[6], ps.hps[7], nwarps, ld);
-        __syncthreads();
+      BoundaryProg<kMode> bp;
+      if (any_boundary) {
+        sc = ps.sched[6][wid];
+        if (sc.z) bp.load(x, make_uint2(sc.x, sc.y), (int)sc.w);
+      }
+      __syncthreads();
+      UFE_TM_SUB(kTmColour0 + 4);
+      UFE_TM(kTmColour);
+      if (wid == nwarps - 1 - nfetch) halo_arrive<kM>(a, t, ps, G);   // (a warp with little else to do)
+      UFE_TM(kTmArrive);
+      if (any_boundary) {
+        // edge rows, then the corners, which average edge rows among others
+        auto boundary = [&](unsigned end) {
+          while (sc.z && sc.w < end) {
+            bp.update(a, x, (int)sc.w, ld);
+            sc.w += (unsigned)nwarps;
+            if (--sc.z) bp.load(x, ps.tab[sc.w / kU], (int)sc.w);
+          }
+          __syncthreads();
+        };
+        boundary((unsigned)(kU * (ps.hps[6] - ps.hps[0])));
+        if (any_corners) boundary(~0u);
       }
       // the exchange buffers move on
-      xin = a.hxch + (size_t)turn * a.xch_stride;
+      xin = x.xout - ex_first;
       turn = turn == kXchBufs - 1 ? 0 : turn + 1;
-      x.xout = a.hxch + (size_t)turn * a.xch_stride + (size_t)ps.ex0 * (kM ? 2 : 4);
+      x.xout = (turn == 0 ? a.hxch : xin + a.xch_stride) + ex_first;
       UFE_TM(kTmBoundary);
       int act = ps.act[G & 1];
-      if (act < 0) return false;
       const bool refold_now = kM && --until_refold == 0;
-      if (refold_now) until_refold = a.refold;
       synced = false;
       last_G = G;
+      if (__builtin_expect(act == 0 && sweeps != a.max_inner && !refold_now, 1)) {
+        UFE_TM(kTmOther);
+        continue;
+      }
+      if (act < 0) return false;
+      if (refold_now) until_refold = a.refold;
       if (act != 0) {
         last_G = G - 1u;
         if constexpr (!kM) {
