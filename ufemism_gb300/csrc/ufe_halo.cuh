@@ -586,7 +586,7 @@ __device__ void halo_refresh(const SsaArgs &a, const HaloSmem &ps, unsigned char
           ++n;
         }
         const double2 u0 = a.UV[g];
-        const double rn = n > 0 ? 1.0 / (double)n : 0.0;
+        const double rn = ps.rcp_n[n];
         *dat = make_float4((float)(sx * rn - u0.x), (float)(sy * rn - u0.y), (float)rn, 0.0f);
       }
     } else if (!boundary) {
@@ -734,7 +734,7 @@ __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
     ++it;
     // N_prev <- N, then the new viscosity into N
     { double *q = N; N = Nprev; Nprev = q; }
-    phase_viscosity(a, t, N, Nprev, kM && a.fp32_visc);
+    phase_viscosity(a, t, N, Nprev, kM && a.fp32_visc, it == 1);
     UFE_GRID_SYNC();
     const double RN = final_rn(a, t);
     if (leader) { ctl->picard_iterations = it; ctl->last_RN = RN; }
@@ -742,7 +742,7 @@ __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
     phase_coefficients<kMode>(a, t);
     UFE_GRID_SYNC();
     if (kM) {
-      phase_defect(a, t);
+      phase_defect<true>(a, t);
       UFE_GRID_SYNC();
     }
     int sweeps = 0;
@@ -879,7 +879,7 @@ __device__ bool solve_member_halo(const SsaArgs &a, Team &t) {
       } else if (refold_now) {
         fold();
         UFE_GRID_SYNC();
-        phase_defect(a, t);
+        phase_defect<true>(a, t);
         UFE_GRID_SYNC();
         halo_refresh<kMode>(a, ps, stage);
       }
