@@ -17,8 +17,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # Build variants: the product library; a profiling build whose persistent solver records
-# per-phase SM-cycle totals (ufe_debug_phase_cycles); builds whose mixed sweeps decide
-# convergence two sweeps late (for measuring the lag). UFE_BUILD_VARIANT selects the one that
+# per-phase SM-cycle totals (ufe_debug_phase_cycles); builds whose phased mixed sweeps
+# decide convergence two sweeps late (for measuring the lag). UFE_BUILD_VARIANT selects the one that
 # ufemism_gb300._native loads.
 VARIANTS = {"": [], "phase_timers": ["-DUFE_PHASE_TIMERS=1"], "lag2": ["-DUFE_MIXED_LAG=2"],
             "lag2_phase_timers": ["-DUFE_MIXED_LAG=2", "-DUFE_PHASE_TIMERS=1"]}

@@ -53,7 +53,7 @@ inline SiaLevels sia_levels(const ufe_params *p) {
 // One thread per Ac edge. At 2 FP64 lanes a clock per SM the arithmetic, not the 2 * 8 * nZ bytes per
 // edge, bounds this kernel: six FP64 instructions per level (the level constants come from the
 // host, the sums are fused, the cut-off compares bits) where the direct form takes fifteen. 100k
-// vertices (285k edges, 15 levels): 124 -> 47 us, of which 11 are the bytes at the copy rate.
+// vertices (306k edges, 15 levels): 142 -> 57 us, of which 11 are the bytes at the copy rate; 1k: 26 -> 7.7.
 template <int NZ>
 __global__ void __launch_bounds__(64) k_sia_edges(int nAc, int nZ_rt, const int *__restrict__ mask,
                                                   const double *__restrict__ H, const double *__restrict__ sx,
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(64) k_sia_edges(int nAc, int nZ_rt, const int 
 
 // map_Ac_to_Aa: d_Aa(vi) = sum_ci d_Ac(iAci(vi,ci)) / nC(vi), in ci order; one thread per vertex and
 // field (blockIdx.y), each quotient correctly rounded from 1 / nC (divide_by): 3 FP64 instructions
-// where a division takes about 20. 1k vertices: 25 -> 4 us; 100k: 98 -> 25 us.
+// where a division takes about 20. 1k vertices: 46 -> 6 us; 100k: 138 -> 24 us.
 __global__ void __launch_bounds__(128) k_ac_to_aa3(int nV, const int *__restrict__ nC, const int *__restrict__ iAci,
                                                   const double *__restrict__ a0, const double *__restrict__ a1,
                                                   const double *__restrict__ a2, double *__restrict__ b0,

@@ -166,7 +166,7 @@ constexpr int kMaxKrylovRestart = 1000;   // largest GMRES restart length of the
 // Threads per CTA of the halo sweeps: 128 registers hold a slice's program across a barrier. On
 // the 200k dome a mixed sweep measured 18.1 us with 1024 threads (64 registers, spilled), 13.7 with
 // 512 and 18.0 with 256; at 16k vertices 8.6, 5.1 and 5.0 (since then the row updates were shortened
-// and the warps' schedules tabulated, which left 11.4 and 3.4 at 512).
+// and the warps' schedules tabulated, which left 11.0 and 3.3 at 512).
 constexpr int kHaloBlock = 512;
 
 // Per-phase timers of the persistent solver (profiling build only, -DUFE_PHASE_TIMERS=1):
@@ -1492,7 +1492,7 @@ __global__ void k_krylov_sub(int n, const double *x, const double *mu, double *y
 // Dot products of up to eight vectors with w over a block's elements: a thread's eight partial sums
 // are loaded together and go through shared memory, where a warp sums one vector (12 FP64
 // additions in a row, 64 cycles each, against 5 per vector and warp in turn). Fixed order. 16k
-// vertices, 17 vectors: 22 -> 12 us.
+// vertices, 17 vectors: 21.7 us -> 15.5 with the subtraction of the pass before in the same launch.
 constexpr int kKrylovThreads = 256, kKrylovChunk = 8;
 __device__ __forceinline__ void krylov_chunk_dots(int n, int nvec, const double *V, size_t ld, const double *w, double *out,
                                                   double (*sacc)[kKrylovThreads]) {
@@ -2569,8 +2569,8 @@ double member_work(int rows, int T, int block) {
 // With the default packing: CTAs that are left when every member has its team at once go to the
 // members expected to take longest (a batch ends with its slowest member), a team growing by the
 // sizes 1, 2, 3, 4, 6, 8, 12, ... The estimate of a solve: rows^0.75 sweeps (184, 324, 876 and 3129
-// on domes of 284, 996, 3336 and 15984 vertices), each 3.4 us and 1 us per 700 rows of a CTA
-// (mixed; 12.1 us at 5,400 rows plus their halo).
+// on domes of 284, 996, 3336 and 15984 vertices), each 3.4 us and 1 us per 700 rows of a CTA (it only
+// ranks members; a single mixed solve's sweep takes 2.8 us at 128 rows a CTA, 11.0 at 5,400 and their halo).
 void spread_teams(const int32_t *rows, int n, int resident, int32_t *team) {
   auto next = [](int t) { return (t & (t - 1)) == 0 ? (t < 2 ? t + 1 : t / 2 * 3) : t / 3 * 4; };
   auto time = [&](int m) { return std::pow((double)rows[m], 0.75) * (3.4 + (double)rows[m] / team[m] / 700.0); };
