@@ -1,0 +1,101 @@
+"""Result arrays from recycled host memory when meshes come and go (no GPU): closing one leaves the
+other meshes' blocks, the next mesh's first results find them, and what is kept is bounded."""
+import gc
+
+import numpy as np
+import pytest
+
+from ufemism_gb300 import api
+
+
+class _Library:
+    """Stands in for the native library where a handle is only closed."""
+
+    def ufe_mesh_destroy(self, h):
+        return 0
+
+    def ufe_batch_destroy(self, h):
+        return 0
+
+
+def handle(kind):
+    h = kind.__new__(kind)
+    h._h = 1
+    api._pool.opened()
+    return h
+
+
+@pytest.fixture
+def pool(monkeypatch):
+    p = api._HostPool(limit=64 << 20, rest=16 << 20)
+    monkeypatch.setattr(api, "_pool", p)
+    monkeypatch.setattr(api.nat, "load", lambda: _Library())
+    return p
+
+
+@pytest.mark.parametrize("kind", [api.DeviceMesh, api.Batch])
+@pytest.mark.parametrize("by_collection", [False, True])
+def test_closing_a_handle_leaves_the_others_blocks(pool, kind, by_collection):
+    kept, other = handle(api.DeviceMesh), handle(kind)
+    used, idle = pool.array(200000), pool.array(300000)
+    where = {used.ctypes.data, idle.ctypes.data}
+    del idle
+    gc.collect()
+    if by_collection:
+        del other
+        gc.collect()
+    else:
+        other.close()
+    del used   # in use when the other handle was closed
+    gc.collect()
+    assert {a.ctypes.data for a in [pool.array(200000), pool.array(300000)]} == where
+    kept.close()
+
+
+@pytest.mark.parametrize("factor", [0.8, 1.0])
+def test_the_next_mesh_finds_the_blocks_of_the_last(pool, factor):
+    mesh = handle(api.DeviceMesh)
+    a = pool.group([(100000, 4), 100000, 50000])
+    where = min(x.ctypes.data for x in a)
+    del a
+    mesh.close()   # the only one
+    gc.collect()
+    handle(api.DeviceMesh)
+    n = int(100000 * factor)
+    assert min(x.ctypes.data for x in pool.group([(n, 4), n, n // 2])) == where
+
+
+def test_idle_memory_after_the_last_handle_is_bounded(pool):
+    mesh, batch = handle(api.DeviceMesh), handle(api.Batch)
+    arrays = [pool.array(1 << 20) for _ in range(12)]   # 8 MiB each
+    last = arrays[-1].ctypes.data
+    for _ in range(12):
+        arrays.pop(0)
+    gc.collect()
+    assert 16 << 20 < pool._bytes <= 64 << 20
+    mesh.close()
+    assert 16 << 20 < pool._bytes
+    batch.close()
+    assert 0 < pool._bytes <= 16 << 20
+    assert pool.array(1 << 20).ctypes.data == last   # the blocks used last are the ones kept
+
+
+def test_a_block_beyond_the_limit_leaves_the_others(pool):
+    mesh = handle(api.DeviceMesh)
+    a = pool.array(1 << 20)
+    where = a.ctypes.data
+    del a
+    b = pool.array(16 << 20)   # 128 MiB
+    del b
+    gc.collect()
+    assert pool._bytes == 8 << 20 and pool.array(1 << 20).ctypes.data == where
+    mesh.close()
+
+
+def test_a_handle_collected_inside_the_pool_does_not_wait_for_itself(pool):
+    mesh, array = handle(api.DeviceMesh), pool.array(100000)
+    with pool._lock:   # a collection in the middle of the pool's work
+        del mesh, array
+        gc.collect()
+    np.testing.assert_array_equal(pool.zeros(100000), 0.0)
+    assert pool._open == 0

@@ -8,6 +8,7 @@ through the C-ABI; nothing here computes a solve on the CPU.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as ct
 import threading
 from dataclasses import dataclass, field
@@ -24,19 +25,25 @@ class _HostPool:
     """Host memory of results that have been dropped, for the next results.
 
     A fresh result array costs its page faults (about 50 us per MB on the GB300's host, against
-    6 us per MB for the copy from the device), so blocks of a page or more are handed out again
-    once no array or view uses them. A block belongs to the array it backs until that array, and
-    every view of it, is gone (the lease is the array's buffer). At most ``limit`` idle bytes are
-    kept; blocks beyond that, and on ``release`` (when a mesh or a batch is closed) all idle ones and
-    those then in use once they are dropped, go back to the allocator. Safe with several threads.
+    6 us per MB for the copy from the device) and the GPU's first access to its pages (10 to 20 us per
+    64 KiB), so blocks of a page or more are handed out again once no array or view uses them. A
+    block belongs to the array it backs until that array, and every view of it, is gone (the lease
+    is the array's buffer). It serves requests of down to half its size, so that a model that has
+    remeshed finds its blocks again. At most ``limit`` idle bytes are kept, those used last, and at
+    most ``rest`` once the last mesh or batch is closed; ``release`` gives the allocator all idle blocks, and
+    those then in use once they are dropped. Safe with several threads.
     """
 
-    def __init__(self, limit: int = 512 << 20, smallest: int = 64 << 10):
-        self.limit, self.smallest = limit, smallest
-        self._idle: dict = {}
+    def __init__(self, limit: int = 512 << 20, smallest: int = 64 << 10, rest: int = 128 << 20):
+        self.limit, self.smallest, self.rest = limit, smallest, rest
+        self._idle: list = []   # idle blocks, the longest unused first
         self._bytes = 0
-        self._age = 0   # releases so far: a block leased before one is not kept when it comes back
-        self._lock = threading.RLock()   # a lease may end (in a collection) while its thread holds the lock
+        self._age = 0    # releases so far: a block leased before one is not kept when it comes back
+        self._open = 0   # meshes and batches
+        self._lock = threading.Lock()
+        # blocks on their way back, None for a closed handle: both may come from a collection while its
+        # thread holds the lock
+        self._returned: collections.deque = collections.deque()
 
     def array(self, shape, dtype=np.float64, order: str = "C"):
         """An uninitialised array."""
@@ -46,12 +53,14 @@ class _HostPool:
         if nbytes < self.smallest:
             return np.empty(shape, dtype, order=order)
         size = -(-nbytes // self.smallest) * self.smallest
+        self._settle()
         with self._lock:
-            blocks = self._idle.get(size)
-            block = blocks.pop() if blocks else None
+            fits = [(b.size, -i) for i, b in enumerate(self._idle) if size <= b.size <= 2 * size]
+            block = self._idle.pop(-min(fits)[1]) if fits else None   # the tightest, of those the one used last
             if block is not None:
-                self._bytes -= size
+                self._bytes -= block.size
             age = self._age
+        self._settle()
         if block is None:
             block = np.empty(size, np.uint8)
         return np.frombuffer(_Lease(self, block, age), dtype, nbytes // dtype.itemsize).reshape(shape, order=order)
@@ -81,16 +90,43 @@ class _HostPool:
         return a
 
     def give_back(self, block, age):
+        self._returned.append((block, age))
+        self._settle()
+
+    def _settle(self):
+        """Take in what was returned, unless the lock is held: its holder does this when it is done."""
+        while self._returned and self._lock.acquire(blocking=False):
+            try:
+                while self._returned:
+                    item = self._returned.popleft()
+                    if item is None:
+                        self._open -= 1
+                    elif item[1] == self._age and item[0].size <= self.limit:
+                        self._idle.append(item[0])
+                        self._bytes += item[0].size
+                    most = self.limit if self._open > 0 else min(self.limit, self.rest)
+                    while self._bytes > most:
+                        self._bytes -= self._idle.pop(0).size
+            finally:
+                self._lock.release()
+
+    def opened(self):
+        """A mesh or batch was created."""
         with self._lock:
-            if age == self._age and self._bytes + block.size <= self.limit:
-                self._idle.setdefault(block.size, []).append(block)
-                self._bytes += block.size
+            self._open += 1
+        self._settle()
+
+    def closed(self):
+        """A mesh or batch was closed; its blocks serve the others, and the next one's first results."""
+        self._returned.append(None)
+        self._settle()
 
     def release(self):
         with self._lock:
             self._idle.clear()
             self._bytes = 0
             self._age += 1
+        self._settle()
 
 
 class _Lease:
@@ -299,6 +335,7 @@ class DeviceMesh:
         if rc != nat.UFE_OK:
             raise nat.UfeError(rc, "ufe_mesh_create")
         self._h = h   # the library copied everything it needs from ``keep``
+        _pool.opened()
 
     @property
     def handle(self):
@@ -312,7 +349,7 @@ class DeviceMesh:
         if getattr(self, "_h", None):
             nat.load().ufe_mesh_destroy(self._h)
             self._h = None
-            _pool.release()   # the idle blocks have this mesh's sizes
+            _pool.closed()
 
     def __del__(self):
         try:
@@ -659,6 +696,7 @@ class Batch:
         if rc != nat.UFE_OK:
             raise nat.UfeError(rc, "ufe_batch_create")
         self._h = h
+        _pool.opened()
         self.n = n
 
     def upload(self, i: int, fields: dict, params: dict, warm: dict | None = None, buffers: dict | None = None):
@@ -711,7 +749,7 @@ class Batch:
         if getattr(self, "_h", None):
             nat.load().ufe_batch_destroy(self._h)
             self._h = None
-            _pool.release()
+            _pool.closed()
 
     def __del__(self):
         try:
