@@ -99,3 +99,23 @@ def test_a_handle_collected_inside_the_pool_does_not_wait_for_itself(pool):
         gc.collect()
     np.testing.assert_array_equal(pool.zeros(100000), 0.0)
     assert pool._open == 0
+
+
+def test_a_lease_is_a_numpy_array_and_ends_once():
+    """No Python-level buffer method, which the interpreter knows from 3.12 on only; the lease ends
+    with the last view, also when that was made from a base of the array."""
+    pool = api._HostPool()
+    assert "__buffer__" not in vars(api._Lease)
+    a = pool.array((5000, 20), order="F")
+    assert type(a) is np.ndarray
+    chain, x = [], a
+    while isinstance(x, np.ndarray):
+        chain.append(x)
+        x = x.base
+    views = [c[1:] for c in chain] + [c.view() for c in chain]
+    del a, chain, x
+    while views:
+        assert pool._bytes == 0
+        views.pop()
+        gc.collect()
+    assert pool._bytes == 13 << 16

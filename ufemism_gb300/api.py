@@ -63,7 +63,10 @@ class _HostPool:
         self._settle()
         if block is None:
             block = np.empty(size, np.uint8)
-        return np.frombuffer(_Lease(self, block, age), dtype, nbytes // dtype.itemsize).reshape(shape, order=order)
+        # (over a ctypes buffer: numpy would take an array's memory, and not the lease, as its views' base)
+        lease = _Lease((nbytes // dtype.itemsize,), dtype, buffer=(ct.c_char * block.size).from_buffer(block))
+        lease._use = (self, block, age)
+        return lease.view(np.ndarray).reshape(shape, order=order)
 
     def group(self, shapes, dtype=np.float64, order: str = "C", most: int = 16 << 20):
         """Uninitialised arrays of the given shapes, one after the other in blocks of at most ``most``
@@ -129,17 +132,15 @@ class _HostPool:
         self._settle()
 
 
-class _Lease:
-    """One array's use of a pool block (the buffer that the array is made from)."""
-
-    def __init__(self, pool, block, age):
-        self._pool, self._block, self._age = pool, block, age
-
-    def __buffer__(self, flags):
-        return memoryview(self._block)
+class _Lease(np.ndarray):
+    """One array's use of a pool block: the base of the array that the caller gets, which every view of
+    that keeps. (A class with a Python-level buffer method would do only from Python 3.12 on.)"""
 
     def __del__(self):
-        self._pool.give_back(self._block, self._age)
+        use = self.__dict__.pop("_use", None)   # (a view of the lease itself has none)
+        if use is not None:
+            pool, block, age = use
+            pool.give_back(block, age)
 
 
 _pool = _HostPool()
