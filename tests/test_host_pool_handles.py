@@ -1,6 +1,7 @@
 """Result arrays from recycled host memory when meshes come and go (no GPU): closing one leaves the
 other meshes' blocks, the next mesh's first results find them, and what is kept is bounded."""
 import gc
+import tracemalloc
 
 import numpy as np
 import pytest
@@ -119,3 +120,46 @@ def test_a_lease_is_a_numpy_array_and_ends_once():
         views.pop()
         gc.collect()
     assert pool._bytes == 13 << 16
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.int32])
+@pytest.mark.parametrize("keep", [0, 2, 5])
+def test_a_kept_field_keeps_little_else(keep, dtype):
+    """The fields of a result lie one after the other, yet a caller that keeps one field of each of
+    many results keeps about these fields' memory (and the other fields are whole and apart)."""
+    pool = api._HostPool()
+    shapes = [(40000,), (20000, 2), (60000,), (7, 3000), (0,), (60001,)]
+    tracemalloc.start()
+    kept, biggest = [], 0
+    for k in range(60):
+        r = pool.group(shapes, dtype, "F")
+        spans = sorted((a.ctypes.data, a.ctypes.data + a.nbytes) for a in r if a.size)
+        assert all(x[1] <= y[0] for x, y in zip(spans, spans[1:]))
+        assert [a.shape for a in r] == shapes and all(a.flags.f_contiguous for a in r)
+        if k == 0:
+            assert all(x[1] == y[0] for x, y in zip(spans, spans[1:]))
+        for a in r:
+            a[...] = k
+        biggest = sum(a.nbytes for a in r)
+        kept.append(r[keep])
+        del r, a
+    assert all(np.all(a == k) for k, a in enumerate(kept))
+    assert tracemalloc.get_traced_memory()[0] < 1.5 * sum(a.nbytes for a in kept) + 3 * biggest
+    tracemalloc.stop()
+    del kept
+    gc.collect()
+    assert not pool._partial and pool._bytes == sum(b.size for b in pool._idle)
+
+
+def test_ranges_join_again_in_any_order():
+    rng = np.random.default_rng(5)
+    block = api._Block(4096, 0)
+    for _ in range(50):
+        cuts = np.unique(np.concatenate([[0, 4096], rng.integers(1, 4096, 9)]))
+        ranges = [(int(a), int(b)) for a, b in zip(cuts, cuts[1:])]
+        for k in rng.permutation(len(ranges)):
+            block.take(*ranges[k])
+        assert block.free == []
+        for k in rng.permutation(len(ranges)):
+            block.give(*ranges[k])
+        assert block.free == [(0, 4096)]

@@ -8,8 +8,10 @@ through the C-ABI; nothing here computes a solve on the CPU.
 """
 from __future__ import annotations
 
+import bisect
 import collections
 import ctypes as ct
+import math
 import threading
 from dataclasses import dataclass, field
 
@@ -21,68 +23,89 @@ ZETA_DEFAULT = np.array([0.00, 0.10, 0.20, 0.30, 0.40, 0.50, 0.60, 0.70, 0.80, 0
                          0.925, 0.95, 0.975, 0.99, 1.00])  # configuration_module.f90:124-126
 
 
+class _Block:
+    """Memory that arrays are made from; ``free``: its ranges that no array has, in order."""
+
+    def __init__(self, size: int, age: int):
+        self.memory = np.empty(size, np.uint8)
+        # (over a ctypes buffer: numpy would take an array's memory, and not the lease, as its views' base)
+        self.buffer = (ct.c_char * size).from_buffer(self.memory)
+        self.size, self.age, self.free = size, age, [(0, size)]
+
+    def take(self, start: int, end: int):
+        k = bisect.bisect_right(self.free, (start, self.size)) - 1
+        a, e = self.free[k]
+        self.free[k:k + 1] = [r for r in ((a, start), (end, e)) if r[0] < r[1]]
+
+    def give(self, start: int, end: int):
+        k = bisect.bisect_left(self.free, (start, end))
+        if k < len(self.free) and self.free[k][0] == end:
+            end = self.free.pop(k)[1]
+        if k > 0 and self.free[k - 1][1] == start:
+            k -= 1
+            start = self.free.pop(k)[0]
+        self.free.insert(k, (start, end))
+
+
 class _HostPool:
     """Host memory of results that have been dropped, for the next results.
 
     A fresh result array costs its page faults (about 50 us per MB on the GB300's host, against
     6 us per MB for the copy from the device) and the GPU's first access to its pages (10 to 20 us per
-    64 KiB), so blocks of a page or more are handed out again once no array or view uses them. A
-    block belongs to the array it backs until that array, and every view of it, is gone (the lease
-    is the array's buffer). It serves requests of down to half its size, so that a model that has
-    remeshed finds its blocks again. At most ``limit`` idle bytes are kept, those used last, and at
-    most ``rest`` once the last mesh or batch is closed; ``release`` gives the allocator all idle blocks, and
-    those then in use once they are dropped. Safe with several threads.
+    64 KiB), so memory of a page or more is handed out again once no array or view uses it. Blocks
+    hold the arrays of one request; each array has a range of its own (the lease, its base), which is
+    free again when that array, and every view of it, is gone, also while others of the block are kept:
+    a caller that keeps one field of each result keeps little else. Idle blocks serve requests of down
+    to half their size, so that a model that has remeshed finds its blocks again. At most ``limit`` idle
+    bytes are kept, those used last, and at most ``rest`` once the last mesh or batch is closed; ``release``
+    gives the allocator all idle blocks, and those then in use once they are dropped. Safe with
+    several threads.
     """
+
+    _ALIGN = 64
 
     def __init__(self, limit: int = 512 << 20, smallest: int = 64 << 10, rest: int = 128 << 20):
         self.limit, self.smallest, self.rest = limit, smallest, rest
-        self._idle: list = []   # idle blocks, the longest unused first
-        self._bytes = 0
-        self._age = 0    # releases so far: a block leased before one is not kept when it comes back
+        self._idle: list = []     # blocks without an array, the longest unused first
+        self._partial: list = []  # blocks of which arrays have a part
+        self._bytes = 0           # of the idle blocks
+        self._age = 0    # releases so far: a block of before one is not used again
         self._open = 0   # meshes and batches
         self._lock = threading.Lock()
-        # blocks on their way back, None for a closed handle: both may come from a collection while its
+        # ranges on their way back, None for a closed handle: both may come from a collection while its
         # thread holds the lock
         self._returned: collections.deque = collections.deque()
 
     def array(self, shape, dtype=np.float64, order: str = "C"):
         """An uninitialised array."""
-        shape = (shape,) if np.isscalar(shape) else tuple(shape)
-        dtype = np.dtype(dtype)
-        nbytes = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
-        if nbytes < self.smallest:
-            return np.empty(shape, dtype, order=order)
-        size = -(-nbytes // self.smallest) * self.smallest
-        self._settle()
-        with self._lock:
-            fits = [(b.size, -i) for i, b in enumerate(self._idle) if size <= b.size <= 2 * size]
-            block = self._idle.pop(-min(fits)[1]) if fits else None   # the tightest, of those the one used last
-            if block is not None:
-                self._bytes -= block.size
-            age = self._age
-        self._settle()
-        if block is None:
-            block = np.empty(size, np.uint8)
-        # (over a ctypes buffer: numpy would take an array's memory, and not the lease, as its views' base)
-        lease = _Lease((nbytes // dtype.itemsize,), dtype, buffer=(ct.c_char * block.size).from_buffer(block))
-        lease._use = (self, block, age)
-        return lease.view(np.ndarray).reshape(shape, order=order)
+        return self.group([shape], dtype, order)[0]
 
     def group(self, shapes, dtype=np.float64, order: str = "C", most: int = 16 << 20):
-        """Uninitialised arrays of the given shapes, one after the other in blocks of at most ``most``
+        """Uninitialised arrays of the given shapes, one after the other in runs of at most ``most``
         bytes (where one array is no larger): results in the order in which the library keeps them on
         the device come back in few copies. Larger blocks the allocator would take fresh from the
         system each time."""
+        dtype = np.dtype(dtype)
         shapes = [(s,) if np.isscalar(s) else tuple(s) for s in shapes]
-        sizes = [int(np.prod(s, dtype=np.int64)) for s in shapes]
-        out, i, limit = [], 0, most // np.dtype(dtype).itemsize
+        sizes = [math.prod(map(int, s)) * dtype.itemsize for s in shapes]
+        out, i = [], 0
         while i < len(sizes):
             n, k = sizes[i], i + 1
-            while k < len(sizes) and n + sizes[k] <= limit:
+            while k < len(sizes) and n + sizes[k] <= most:
                 n, k = n + sizes[k], k + 1
-            flat, at = self.array(n, dtype), 0
+            if n < self.smallest:
+                small, at = np.empty(n, np.uint8), 0
+            else:
+                block, at, k = self._place(sizes[i:k], n)
+                k += i
             for shape, size in zip(shapes[i:k], sizes[i:k]):
-                out.append(flat[at:at + size].reshape(shape, order=order))
+                if n < self.smallest:
+                    part = small[at:at + size].view(dtype)
+                else:
+                    lease = _Lease((size // dtype.itemsize,), dtype, buffer=block.buffer, offset=at)
+                    lease._use = (self, block, at, at + size)
+                    part = lease.view(np.ndarray)
+                out.append(part if len(shape) == 1 else part.reshape(shape, order=order))
                 at += size
             i = k
         return out
@@ -92,8 +115,51 @@ class _HostPool:
         a.fill(0)
         return a
 
-    def give_back(self, block, age):
-        self._returned.append((block, age))
+    def _place(self, sizes: list, total: int):
+        """Room for the first k of arrays of these sizes, one after the other: (block, start, k).
+
+        The tightest free range that holds them all; else as many as go into the largest one, if that
+        is a quarter of them (smaller ranges stay free, so at least three quarters of a block serve
+        before another is taken); else a new block."""
+        self._settle()
+        with self._lock:
+            tight = roomy = None
+            for b in self._partial + self._idle[::-1]:
+                whole = len(b.free) == 1 and b.free[0] == (0, b.size)
+                if whole and b.size > 2 * total + self.smallest:
+                    continue
+                for start, end in b.free:
+                    start = -(-start // self._ALIGN) * self._ALIGN
+                    room = end - start
+                    if room >= total and (tight is None or room < tight[0]):
+                        tight = room, b, start
+                    if roomy is None or room > roomy[0]:
+                        roomy = room, b, start
+            k, n = len(sizes), total
+            if tight is not None:
+                _, block, start = tight
+            else:
+                block, start = None, 0
+                if roomy is not None:
+                    k = n = 0
+                    while n + sizes[k] <= roomy[0]:
+                        n, k = n + sizes[k], k + 1
+                    if 4 * n >= total:
+                        _, block, start = roomy
+                if block is None:
+                    k, n = len(sizes), total
+                    block = _Block(-(-total // self.smallest) * self.smallest, self._age)
+                    self._partial.append(block)
+            if len(block.free) == 1 and block.free[0] == (0, block.size) and block in self._idle:
+                self._idle.remove(block)
+                self._bytes -= block.size
+                self._partial.append(block)
+            block.take(start, start + n)
+        self._settle()
+        return block, start, k
+
+    def give_back(self, *use):
+        self._returned.append(use)
         self._settle()
 
     def _settle(self):
@@ -101,17 +167,26 @@ class _HostPool:
         while self._returned and self._lock.acquire(blocking=False):
             try:
                 while self._returned:
-                    item = self._returned.popleft()
-                    if item is None:
+                    use = self._returned.popleft()
+                    if use is None:
                         self._open -= 1
-                    elif item[1] == self._age and item[0].size <= self.limit:
-                        self._idle.append(item[0])
-                        self._bytes += item[0].size
+                    else:
+                        self._take_in(*use)
                     most = self.limit if self._open > 0 else min(self.limit, self.rest)
                     while self._bytes > most:
                         self._bytes -= self._idle.pop(0).size
             finally:
                 self._lock.release()
+
+    def _take_in(self, block, start, end):
+        if block.age != self._age:
+            return
+        block.give(start, end)
+        if block.free[0] == (0, block.size):
+            self._partial.remove(block)
+            if block.size <= self.limit:
+                self._idle.append(block)
+                self._bytes += block.size
 
     def opened(self):
         """A mesh or batch was created."""
@@ -127,20 +202,21 @@ class _HostPool:
     def release(self):
         with self._lock:
             self._idle.clear()
+            self._partial.clear()
             self._bytes = 0
             self._age += 1
         self._settle()
 
 
 class _Lease(np.ndarray):
-    """One array's use of a pool block: the base of the array that the caller gets, which every view of
-    that keeps. (A class with a Python-level buffer method would do only from Python 3.12 on.)"""
+    """One array's use of a range of a block: the base of the array that the caller gets, which every
+    view of that keeps. (A class with a Python-level buffer method would do only from Python 3.12 on.)"""
+
+    _use = None   # (of a view of the lease itself)
 
     def __del__(self):
-        use = self.__dict__.pop("_use", None)   # (a view of the lease itself has none)
-        if use is not None:
-            pool, block, age = use
-            pool.give_back(block, age)
+        if self._use is not None:
+            self._use[0].give_back(*self._use[1:])
 
 
 _pool = _HostPool()
