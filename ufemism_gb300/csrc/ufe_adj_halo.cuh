@@ -142,8 +142,9 @@ struct AdjProg {
   }
 };
 
+// A bounded wait's retry (as wait_retry); a limit below a microsecond is looked at on every one.
 __device__ __forceinline__ bool adj_retry(const AdjHaloArgs &a, unsigned &tries, unsigned long long &t0) {
-  if ((++tries & 15u) != 0u) return true;
+  if ((++tries & 15u) != 0u && a.timeout_ns >= 1000) return true;
   if (*(volatile unsigned int *)a.flag) return false;
   const unsigned long long now = globaltimer_ns();
   if (t0 == 0ull) { t0 = now; return true; }

@@ -1574,16 +1574,17 @@ __global__ void __launch_bounds__(kKrylovThreads) k_krylov_pass(int n, int nvec,
     krylov_chunk_dots(n, min(kKrylovChunk, ndots - i0), V + (size_t)i0 * ld, ld, w, next + (size_t)i0 * gridDim.x, sacc);
 }
 
-// v = w / |w| with |w| from its squares' partials; |w| and the sweeps' error flag go to hout.
+// v = w / |w| with |w| from its squares' partials; |w| and the error of the column's sweeps (0: none) go
+// to hout, so that each column's error comes back with its coefficients.
 __global__ void __launch_bounds__(256) k_krylov_normalise(int n, int nblocks, const double *part, const double *w, double *v,
-                                                          double *hout, const unsigned int *flag) {
+                                                          double *hout, const int *err) {
   __shared__ double s;
   krylov_sums(1, nblocks, part, &s);
   if (threadIdx.x == 0) {   // the root and the quotient once per block (about 40 FP64 instructions)
     const double nw = sqrt(s);
     if (blockIdx.x == 0) {
       hout[0] = nw;
-      hout[1] = flag && flag[0] ? (double)(int)flag[1] : 0.0;
+      hout[1] = (double)*err;
     }
     s = nw > 0.0 ? 1.0 / nw : 0.0;
   }
@@ -3534,10 +3535,9 @@ int adj_gmres(Krylov &k, int m, double tol, int max_iter, double *rel, int *iter
       k_krylov_pass<<<kKrylovBlocks, kKrylovThreads, nv * sizeof(double), k.s>>>(k.n, nv, k.V, k.ld, p1, k.w, hd, nv, p2);
       k_krylov_pass<<<kKrylovBlocks, kKrylovThreads, nv * sizeof(double), k.s>>>(k.n, nv, k.V, k.ld, p2, k.w, hd + nv, 0, p1);
       k_krylov_normalise<<<kKrylovBlocks, 256, 0, k.s>>>(k.n, kKrylovBlocks, p1, k.w, k.V + (size_t)nv * k.ld, hd + 2 * nv,
-                                               k.halo ? k.a->halo.flag : nullptr);
+                                               k.halo ? reinterpret_cast<const int *>(k.a->halo.flag + 1) : &k.a->ctl->err);
       e = cuda_status(cudaGetLastError(), "krylov column");
       if (!e) e = cuda_status(cudaMemcpyAsync(hh, hd, (2 * (size_t)nv + 2) * sizeof(double), cudaMemcpyDeviceToHost, k.s), "column D2H");
-      if (!e && !k.halo) e = cuda_status(cudaMemcpyAsync(k.a->ctl_host, k.a->ctl, sizeof(AdjCtl), cudaMemcpyDeviceToHost, k.s), "ctl D2H");
       if (!e) e = cuda_status(cudaEventRecord(k.a->evh[j & 1], k.s), "event");
       return e;
     };
@@ -3557,9 +3557,7 @@ int adj_gmres(Krylov &k, int m, double tol, int max_iter, double *rel, int *iter
       const double *hh = k.a->part_host + (size_t)(j & 1) * (2 * (size_t)kMaxKrylovRestart + 4);
       for (int i = 0; i <= j; ++i) hcol[i] = hh[i] + hh[j + 1 + i];
       const double nw = hh[2 * (j + 1)];
-      const int flag = (int)hh[2 * (j + 1) + 1];
-      if (flag) k.err = flag;
-      if (!k.halo && k.a->ctl_host->err) k.err = k.a->ctl_host->err;
+      k.err = (int)hh[2 * (j + 1) + 1];
       if (k.err) return k.err;
       for (int i = 0; i <= j; ++i) Hm(i, j) = hcol[i];
       Hm(j + 1, j) = nw;
@@ -3706,7 +3704,10 @@ extern "C" int ufe_ssa_vjp(ufe_mesh_h h, const ufe_params *p, const ufe_vjp_para
       k.zero = reinterpret_cast<double2 *>(k.c + n2);
       k.sweeps_per_apply = vp && vp->sweeps_per_iteration > 0 ? vp->sweeps_per_iteration : 8;
       rc = cuda_status(cudaMemsetAsync(k.zero, 0, n2 * sizeof(double), s), "memset zero");
-      if (!rc && !a->halo.tried) {
+      // (UFE_SSA_HALO=0: the phased sweeps, as for the solve)
+      const char *henv = std::getenv("UFE_SSA_HALO");
+      const bool want_halo = !(henv && henv[0] == '0');
+      if (!rc && want_halo && !a->halo.tried) {
         try {
           rc = adj_halo_create(h, a->halo);
         } catch (const std::bad_alloc &) {   // no host memory for the program: the phased sweeps
@@ -3714,9 +3715,10 @@ extern "C" int ufe_ssa_vjp(ufe_mesh_h h, const ufe_params *p, const ufe_vjp_para
           a->halo.ok = false;
         }
       }
-      if (!rc && a->halo.ok) rc = halo_prepare(k);
+      if (!rc && want_halo && a->halo.ok) rc = halo_prepare(k);
       const int max_iter = vp && vp->max_sweeps > 0 ? vp->max_sweeps : 50000;
       if (!rc) rc = adj_gmres(k, restart, tol, max_iter, &k_rel, &k_iters);
+      if (rc) cudaStreamSynchronize(s);   // a column queued ahead writes to the handle's host memory
       k_iters = k.sweeps;
       k_err = k.err;
       if (rc == UFE_DIVERGED) { rc = UFE_OK; k_rel = HUGE_VAL; k_err = UFE_DIVERGED; }
