@@ -51,3 +51,32 @@ def test_wait_timeout_reported_and_handle_usable(solved, halo, restart, monkeypa
     assert rc == 0 and st2["sweeps"] == st["sweeps"]
     for k in GRADIENTS:
         assert np.array_equal(again[k], first[k]), k
+
+
+def test_no_device_memory_for_the_program(monkeypatch):
+    """Where the device has no room for the transposed halo sweeps' program, the phased sweeps run. (The
+    program of this mesh takes about 80 MB; all but 32 MB of the device is taken.)"""
+    api.init(0)
+    m = oracle_aaac("50k")
+    ssa, _, _ = oracle_inputs(m)
+    p = api.default_params(precision=nat.UFE_MIXED)
+    dm = api.DeviceMesh(m)
+    dm.solve_ssa(ssa, p)
+    rng = np.random.default_rng(12)
+    dJ = {k: rng.standard_normal(n) for k, n in (("U_SSA", m.base.nV), ("V_SSA", m.base.nV), ("Ux_SSA_Ac", m.nAc),
+                                                 ("Uy_SSA_Ac", m.nAc))}
+    monkeypatch.setenv("UFE_SSA_HALO", "0")
+    rc0, phased, _ = dm.ssa_vjp(dJ, p)
+    monkeypatch.delenv("UFE_SSA_HALO")
+    assert rc0 == 0
+    torch.cuda.empty_cache()
+    taken = torch.empty(max(0, torch.cuda.mem_get_info()[0] - (32 << 20)), dtype=torch.uint8, device="cuda")
+    try:
+        rc, got, _ = dm.ssa_vjp(dJ, p)
+    finally:
+        del taken
+        torch.cuda.empty_cache()
+    assert rc == 0
+    for k in GRADIENTS:
+        assert np.array_equal(got[k], phased[k]), k
+    dm.close()

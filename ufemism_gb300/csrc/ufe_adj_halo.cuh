@@ -520,8 +520,8 @@ inline bool adj_build_host(int nP, int n_patch, const std::vector<int> &patch_sl
   return o.prog_bytes / 16 < ((size_t)1 << 31);
 }
 
-// Builds and uploads a handle's program; ok stays false where it does not apply (the phased sweeps
-// then run).
+// Builds and uploads a handle's program; ok stays false where it does not apply or the device has no
+// room for it (the phased sweeps then run).
 inline int adj_halo_create(ufe_mesh_h h, AdjHalo &d) {
   d.tried = true;
   const DevMesh &m = h->m;
@@ -558,11 +558,17 @@ inline int adj_halo_create(ufe_mesh_h h, AdjHalo &d) {
   d.n_export = o.hex_ptr.back();
   const size_t xbytes = (size_t)kAdjSweeps * 6 * d.n_export * sizeof(unsigned long long);
   unsigned char *index = nullptr;
-  rc = cuda_status(cudaMalloc(&d.ints, all.size() * sizeof(int)), "adjoint program");
-  if (!rc) rc = cuda_status(cudaMalloc(&d.prog, o.prog_bytes), "adjoint program");
-  if (!rc) rc = cuda_status(cudaMalloc(&d.xch, xbytes + 16), "adjoint exchange");
-  if (!rc) rc = cuda_status(cudaMalloc(&d.flag, 2 * sizeof(unsigned int)), "adjoint flag");
-  if (!rc) rc = cuda_status(cudaMalloc(&index, o.index_bytes.size()), "adjoint program");
+  cudaError_t e = cudaMalloc(&d.ints, all.size() * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&d.prog, o.prog_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&d.xch, xbytes + 16);
+  if (e == cudaSuccess) e = cudaMalloc(&d.flag, 2 * sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMalloc(&index, o.index_bytes.size());
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    d.free_all();
+    return UFE_OK;
+  }
+  rc = cuda_status(e, "adjoint program");
   if (!rc) rc = cuda_status(cudaMemcpyAsync(d.ints, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice, s), "adjoint program");
   if (!rc) rc = cuda_status(cudaMemcpyAsync(index, o.index_bytes.data(), o.index_bytes.size(), cudaMemcpyHostToDevice, s), "adjoint program");
   if (!rc) rc = cuda_status(cudaMemsetAsync(d.xch, 0, xbytes + 16, s), "adjoint exchange");
