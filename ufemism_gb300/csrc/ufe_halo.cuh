@@ -345,7 +345,7 @@ template <> struct Prog<kMixed> {
     const float2 dn = make_float2(fmaf(-omega, ru, di.x), fmaf(-omega, rv, di.y));
     ld[l] = dn;
     if (ex != kNoCol) export_value(x.xout + 2 * ex, x.tag, dn);
-    if ((int)l < x.n_own) mx = fmaxf(mx, fmaxf(fabsf(ru), fabsf(rv)));
+    if ((int)l < x.n_own) mx = max_keep_nan(mx, max_keep_nan(fabsf(ru), fabsf(rv)));
   }
 };
 

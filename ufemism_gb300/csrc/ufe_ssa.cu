@@ -349,6 +349,13 @@ __device__ __forceinline__ unsigned long long abs_bits(double x) {
   return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
 }
 
+// The maximum that keeps NaN (fmaxf drops it): a sweep with NaN rows is neither converged nor diverged.
+__device__ __forceinline__ float max_keep_nan(float a, float b) {
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+  return m;
+}
+
 __device__ __forceinline__ bool is_floating(double Hi, double Hb, double SL) {
   return Hi < divide_by((SL - Hb) * kSeawaterDensity, kIceDensity, 1.0 / kIceDensity);   // general_ice_model_data_module.f90:464-475
 }
@@ -677,7 +684,7 @@ __device__ unsigned long long phase_sweep32(const SsaArgs &a, const PatchSmem &p
     }
     const float ru = fmaf(fmaf(s3, di.y, su) - d.x, r.x, di.x);
     const float rv = fmaf(fmaf(s3, di.x, sv) - d.y, r.y, di.y);
-    mx = fmaxf(mx, fmaxf(fabsf(ru), fabsf(rv)));
+    mx = max_keep_nan(mx, max_keep_nan(fabsf(ru), fabsf(rv)));
     const float2 dn = make_float2(fmaf(-omega, ru, di.x), fmaf(-omega, rv, di.y));
     if (lc.n) ld[p - lc.p0] = dn;
     a.dUV[p] = dn;
