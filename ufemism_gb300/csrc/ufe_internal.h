@@ -248,7 +248,7 @@ __device__ __forceinline__ double divide_by(double a, double b, double r) {
   const double q = a * r;
   const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eq = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
   if (ea - 200u < 1600u && eq - 200u < 1600u) return fma(fma(-q, b, a), r, q);
-  if (((unsigned long long)__double_as_longlong(a) << 1) == 0ull) return q;   // a zero: exact
+  if (((unsigned long long)__double_as_longlong(a) << 1) == 0ull && eq < 0x7ffu) return q;   // a zero (r finite): exact
   return divide_ieee(a, b);
 }
 
