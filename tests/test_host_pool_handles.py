@@ -163,3 +163,31 @@ def test_ranges_join_again_in_any_order():
         for k in rng.permutation(len(ranges)):
             block.give(*ranges[k])
         assert block.free == [(0, 4096)]
+
+
+def test_stale_pages_are_written_in_the_range_only(monkeypatch):
+    monkeypatch.setattr(api.time, "monotonic", iter(range(100)).__next__)   # a second between requests
+    pool = api._HostPool()
+    page = api.mmap.PAGESIZE
+    a = pool.group([16 * page, 16 * page, 16 * page], np.uint8)
+    for x in a:
+        x.fill(7)
+    middle = a.pop(1).ctypes.data
+    b = pool.array(16 * page, np.uint8)
+    assert b.ctypes.data == middle
+    assert np.all(b[::page] == 0) and b[-1] == 0 and np.count_nonzero(b == 0) == 17
+    assert all(np.all(x == 7) for x in a)
+
+
+def test_of_many_blocks_one_of_the_size_is_found():
+    pool = api._HostPool()
+    sizes = [65536 * k for k in range(1, 40)]
+    held = [pool.array(n, np.uint8) for n in sizes]
+    where = [x.ctypes.data for x in held]
+    del held
+    for n, at in reversed(list(zip(sizes, where))):
+        x = pool.array(n, np.uint8)
+        assert x.ctypes.data == at
+        del x
+    pool.release()
+    assert not pool._of_size and not pool._idle
