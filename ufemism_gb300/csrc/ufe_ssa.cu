@@ -2627,11 +2627,20 @@ int plan_batch(const int32_t *rows, int n, const ufe_batch_config &cfg, int resi
     }
     team_of_member[m] = T;
   }
-  if (cfg.team_ctas == 0 && cfg.rows_per_cta == 0) spread_teams(rows, n, resident, team_of_member);
   // Classes: distinct team sizes, largest first.
-  std::vector<int> sizes(team_of_member, team_of_member + n);
-  std::sort(sizes.begin(), sizes.end(), std::greater<int>());
-  sizes.erase(std::unique(sizes.begin(), sizes.end()), sizes.end());
+  auto classes = [&]() {
+    std::vector<int> s(team_of_member, team_of_member + n);
+    std::sort(s.begin(), s.end(), std::greater<int>());
+    s.erase(std::unique(s.begin(), s.end()), s.end());
+    return s;
+  };
+  if (cfg.team_ctas == 0 && cfg.rows_per_cta == 0) {
+    const std::vector<int32_t> packed(team_of_member, team_of_member + n);
+    spread_teams(rows, n, resident, team_of_member);
+    // (more team sizes than there are classes, on devices of a thousand CTAs and more: the packing as it was)
+    if ((int)classes().size() > kMaxClasses) std::copy(packed.begin(), packed.end(), team_of_member);
+  }
+  const std::vector<int> sizes = classes();
   if ((int)sizes.size() > kMaxClasses) { set_error("ufe_batch_plan: too many team sizes"); return UFE_BAD_ARG; }
   const int nc = (int)sizes.size();
   std::vector<double> W(nc, 0.0);
