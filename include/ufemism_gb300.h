@@ -430,8 +430,8 @@ int ufe_batch_upload(ufe_batch_h batch, int32_t member, const ufe_params *params
 /* stats: (n_members) or NULL. Returns the most severe member status. */
 int ufe_batch_run(ufe_batch_h batch, const ufe_params *params, ufe_ssa_stats *stats, ufe_batch_timing *timing);
 int ufe_batch_download(ufe_batch_h batch, int32_t member, ufe_ssa_inout *inout, ufe_ssa_out *out);
-/* Autotuner: times real batches of the given members over the per-CTA packing
- * (rows_per_cta 4096..24576 at 1024-thread CTAs), then the CTA size (512, 256) at the best
+/* Autotuner: times real batches of the given members over the per-CTA packing (rows_per_cta 0,
+ * the default, and 4096..24576 at 1024-thread CTAs), then the CTA size (512, 256) at the best
  * packing, then the neighbouring packings at the best CTA size, and returns the fastest
  * configuration. log (capacity entries) receives one entry
  * per candidate tried. Candidates that cannot hold the members are skipped. */

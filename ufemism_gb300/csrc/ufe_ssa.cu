@@ -3182,8 +3182,8 @@ extern "C" int ufe_ssa_solve_batched(int32_t n, const ufe_mesh_desc *descs, cons
 }
 
 // Autotuner of the batched solve: the per-CTA packing (rows_per_cta, hence the team size of
-// every member) first at 1024-thread CTAs, then the CTA size at the best packing, then the
-// neighbouring packings at the best CTA size. Each
+// every member) first at 1024-thread CTAs, the default one (0: idle CTAs spread) among them, then
+// the CTA size at the best packing, then the neighbouring packings at the best CTA size. Each
 // candidate is a real batch of the caller's members, solved twice (the first run captures
 // the graph); the second run's device time decides.
 extern "C" int ufe_batch_autotune(int32_t n, const ufe_mesh_desc *descs, const ufe_params *p, const ufe_ssa_in *in,
@@ -3192,7 +3192,7 @@ extern "C" int ufe_batch_autotune(int32_t n, const ufe_mesh_desc *descs, const u
   if (!descs || !p || !in || !io || !best || n < 1) { set_error("ufe_batch_autotune: null argument"); return UFE_BAD_ARG; }
   int n_log = 0;
   double best_ms = 1e300;
-  ufe_batch_config best_cfg{0, kDefaultRowsPerCta, 1024, 1};
+  ufe_batch_config best_cfg{0, 0, 1024, 1};
   auto trial = [&](const ufe_batch_config &c) -> int {
     ufe_batch_h b = nullptr;
     int rc = ufe_batch_create(descs, n, &c, &b);
@@ -3218,19 +3218,19 @@ extern "C" int ufe_batch_autotune(int32_t n, const ufe_mesh_desc *descs, const u
     return UFE_OK;
   };
   int rc = UFE_OK;
-  const int packings[] = {4096, 8192, 16384, kMaxRowsPerPatch};
-  const int n_pack = 4;
+  const int packings[] = {0, 4096, 8192, 16384, kMaxRowsPerPatch};
+  const int n_pack = 5;
   for (int R : packings)
     if (!rc) rc = trial(ufe_batch_config{0, R, 1024, 1});
   const int R = best_cfg.rows_per_cta;
   for (int blk : {512, 256})
     if (!rc) rc = trial(ufe_batch_config{0, R, blk, 1});
-  // The packings next to the best one at the best CTA size.
+  // The packings next to the best one at the best CTA size (the default one has none).
   const int blk = best_cfg.block;
-  if (blk != 1024) {
+  if (blk != 1024 && R > 0) {
     const int i = (int)(std::find(packings, packings + n_pack, R) - packings);
     for (int j : {i - 1, i + 1})
-      if (!rc && j >= 0 && j < n_pack) rc = trial(ufe_batch_config{0, packings[j], blk, 1});
+      if (!rc && j >= 1 && j < n_pack) rc = trial(ufe_batch_config{0, packings[j], blk, 1});
   }
   if (log_count) *log_count = n_log;
   if (rc) return rc;
