@@ -912,11 +912,7 @@ __global__ void k_sia3d_uv(const __grid_constant__ Sia3dArgs a) {
     return;
   }
   const double sx = a.dHs_dx[v], sy = a.dHs_dy[v];
-  // (rho g H)^3 with the rounding errors of its products carried (as k_sia_edges)
-  const double x = (kIceDensity * kGrav) * h;
-  const double x2 = x * x, x3 = x2 * x;
-  const double cube = x3 + fma(fma(x, x, -x2), x, fma(x2, x, -x3));
-  const double D0 = (cube * fma(sx, sx, sy * sy)) * (2.0 * h);
+  const double D0 = (cube_carried((kIceDensity * kGrav) * h) * fma(sx, sx, sy * sy)) * (2.0 * h);
   const int nZ = a.nZ;
   double f_hi = a.A[v + (size_t)(nZ - 1) * ld] * a.c[nZ - 1];
   double acc = 0.0;

@@ -271,6 +271,13 @@ __device__ __forceinline__ double reciprocal_rn(double b) {
   return divide_ieee(1.0, b);
 }
 
+// x^3 with the rounding errors of its products carried (below 0.51 ulp); one that overflows is infinite.
+__device__ __forceinline__ double cube_carried(double x) {
+  const double x2 = x * x, x3 = x2 * x;
+  const double c = x3 + fma(fma(x, x, -x2), x, fma(x2, x, -x3));
+  return ((unsigned)__double2hiint(x3) & 0x7ff00000u) == 0x7ff00000u ? x3 : c;
+}
+
 // 1 / n of the small counts that the kernels divide by, rounded to nearest (a kernel parameter).
 struct CountReciprocals {
   double n[kMaxDeg + 1], r[kMaxDeg + 1];   // n as a double, and 1 / n

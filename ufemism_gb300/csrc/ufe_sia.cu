@@ -75,12 +75,8 @@ __global__ void __launch_bounds__(64) k_sia_edges(int nAc, int nZ_rt, const int 
     const double h = H[a];
     const double p = sp[a], o = so[a];
     const double px = sx[a], py = sy[a];
-    // (rho g H)^n * (dHs_dp^2 + dHs_do^2)^((n-1)/2), n = 3: the cube with the rounding errors of
-    // its products carried (below 0.51 ulp), the second power is 1
-    const double x = (kIceDensity * kGrav) * h;
-    const double x2 = x * x, x3 = x2 * x;
-    const double cube = x3 + fma(fma(x, x, -x2), x, fma(x2, x, -x3));
-    const double D0 = (cube * fma(p, p, o * o)) * (2.0 * h);
+    // (rho g H)^n * (dHs_dp^2 + dHs_do^2)^((n-1)/2), n = 3: the second power is 1
+    const double D0 = (cube_carried((kIceDensity * kGrav) * h) * fma(p, p, o * o)) * (2.0 * h);
     // vertical_integrate( m_enh_sia * A_flow * zeta^n ), from the base upwards; the cut-off and the
     // vertical average on the way
     double f_hi = d3[nZ - 1] * lev.c[nZ - 1];
