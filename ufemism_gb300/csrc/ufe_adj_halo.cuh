@@ -336,7 +336,7 @@ __global__ void k_adj_fill(const AdjFill a) {
 struct AdjHalo {
   bool tried = false, ok = false;
   int n_slices = 0, max_local = 0, max_halo = 0, n_export = 0;
-  unsigned tag = 1;                                // next unused tag
+  unsigned tag = 0xffffff00u - 100u;               // next unused tag (near its end, so that every handle passes it early)
   int *ints = nullptr;                             // every index array
   const int *hp_slice = nullptr, *hp_split = nullptr, *slice_b0 = nullptr, *slice_w = nullptr, *hrow_g = nullptr;
   const int *hload_ptr = nullptr, *hload_dev = nullptr, *hload_ex = nullptr, *hex_ptr = nullptr;
