@@ -935,8 +935,8 @@ __global__ void k_sia3d_uv(const __grid_constant__ Sia3dArgs a) {
 // apply_Neumann_boundary_3D on one or two fields (blockIdx.z), one thread per vertex and level: an edge
 // vertex becomes the mean of its non-edge neighbours, a corner (vertices 0..3) the mean of all its
 // neighbours, an edge neighbour among them by its new value, formed again here (same arithmetic),
-// so that edges and corners need one launch. Results go to `out` first (the edge rows read
-// non-edge rows only, which nothing writes).
+// so that edges and corners need one launch (written in place: what is read is no edge row's value,
+// and nothing writes the other rows).
 __device__ __forceinline__ double edge_mean3(const Sia3dArgs &a, const double *d, int v, const CountReciprocals &rc) {
   const size_t ld = a.nV;
   const int n = a.nC[v];

@@ -461,7 +461,8 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
       if (n_own + (int)halo.size() > 65533) { halo_ok = false; break; }
       m.max_local = std::max(m.max_local, n_own + (int)halo.size());
       m.max_halo = std::max(m.max_halo, (int)halo.size());
-      for (int p : halo) hreads[b].push_back(patch_of[orig_of_dev[p]]);
+      if (t_dump_path)
+        for (int p : halo) hreads[b].push_back(patch_of[orig_of_dev[p]]);
       hload_dev.insert(hload_dev.end(), halo.begin(), halo.end());
       hload_ptr.push_back((int)hload_dev.size());
     }
@@ -601,12 +602,12 @@ int mesh_create(const ufe_mesh_desc *d, int n_patch_request, ufe_mesh_h *out) {
     }
     if (halo_ok) {
       hp_slice.push_back((int)hslice_e0.size());   // end of the last patch
-      // the patches that exchange rows (symmetric closure; a check of the layout's consistency)
+      // the patches that exchange rows (symmetric closure; the layout dump's check of its consistency)
       std::vector<std::vector<int>> hs(n_patch);
       for (int b = 0; b < n_patch; ++b)
         for (int q : hreads[b])
           if (q != b) { hs[b].push_back(q); hs[q].push_back(b); }
-      for (int b = 0; b < n_patch; ++b) {
+      for (int b = 0; b < n_patch && t_dump_path; ++b) {
         std::sort(hs[b].begin(), hs[b].end());
         hs[b].erase(std::unique(hs[b].begin(), hs[b].end()), hs[b].end());
         hsync_list.insert(hsync_list.end(), hs[b].begin(), hs[b].end());

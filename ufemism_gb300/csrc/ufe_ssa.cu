@@ -3509,7 +3509,7 @@ int adj_gmres(Krylov &k, int m, double tol, int max_iter, double *rel, int *iter
     k_krylov_load<<<gp, 256, 0, k.s>>>(k.nP, nullptr, k.a->alpha, k.a->mu, k.a->s);
     return cuda_status(cudaGetLastError(), "k_krylov_load");
   }
-  std::vector<double> H((size_t)(m + 1) * m, 0.0), cs(m), sn(m), gv(m + 1), hcol(m + 1), h2(m + 1), y(m);
+  std::vector<double> H((size_t)(m + 1) * m, 0.0), cs(m), sn(m), gv(m + 1), hcol(m + 1), y(m);
   auto Hm = [&](int i, int j) -> double & { return H[(size_t)j * (m + 1) + i]; };
   int total = 0;
   double res = 1.0, cycle_start = 1.0;
