@@ -1,6 +1,8 @@
 """Result arrays from recycled host memory when meshes come and go (no GPU): closing one leaves the
 other meshes' blocks, the next mesh's first results find them, and what is kept is bounded."""
 import gc
+import random
+import threading
 import tracemalloc
 
 import numpy as np
@@ -191,3 +193,39 @@ def test_of_many_blocks_one_of_the_size_is_found():
         del x
     pool.release()
     assert not pool._of_size and not pool._idle
+
+
+def test_threads_hold_and_drop_fields_in_any_order():
+    """Random groups (empty and small arrays among them), some fields kept, collections and releases in
+    between: every field keeps its values while it is held, and the books balance in the end."""
+    pool = api._HostPool(limit=24 << 20, rest=8 << 20)
+    bad = []
+
+    def work(k):
+        rng, held = random.Random(k), []
+        try:
+            for i in range(300):
+                shapes = [rng.choice([1000, 9000, 20000, 70001, (300, 100), (0,), 5]) for _ in range(rng.randint(1, 8))]
+                fields = pool.group(shapes, rng.choice([np.float64, np.int32]), rng.choice("CF"))
+                for a in fields:
+                    a[...] = 1000 * k + i
+                held.append((1000 * k + i, rng.sample(fields, rng.randint(0, len(fields)))))
+                if len(held) > 12:
+                    tag, kept = held.pop(rng.randrange(len(held)))
+                    bad.extend(tag for a in kept if not np.all(a == tag))
+                if rng.random() < 0.01:
+                    pool.release()
+                if rng.random() < 0.02:
+                    gc.collect()
+            bad.extend(tag for tag, kept in held if not all(np.all(a == tag) for a in kept))
+        except Exception as e:
+            bad.append(e)
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    gc.collect()
+    assert not bad
+    assert not pool._partial and pool._bytes == sum(b.size for b in pool._idle) <= 8 << 20
+    assert sum(map(len, pool._of_size.values())) == len(pool._idle)
+    assert all(b.free == [(0, b.size)] for b in pool._idle)

@@ -109,7 +109,9 @@ class _HostPool:
                 block, at, k = self._place(sizes[i:k], n)
                 k += i
             for shape, size in zip(shapes[i:k], sizes[i:k]):
-                if n < self.smallest:
+                if size == 0:   # (no range to return)
+                    part = np.empty(0, dtype)
+                elif n < self.smallest:
                     part = small[at:at + size].view(dtype)
                 else:
                     lease = _Lease((size // dtype.itemsize,), dtype, buffer=block.buffer, offset=at)
