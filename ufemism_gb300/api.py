@@ -69,8 +69,9 @@ class _HostPool:
     _ALIGN = 64
     # Seconds after which a block's pages are written to before the GPU gets them. Its first access to
     # a page that the CPU has not written for a while (or ever) costs 10 to 20 us, the CPU's 0.1: the results
-    # of a geometry update at 100k vertices (70 MB), a second of other work after the last ones, take 4.5
-    # ms instead of 10 to 33. In a loop of calls it would cost 3% (0.05 ms of 1.5).
+    # of a geometry update at 100k vertices (70 MB), a second of other work after the last ones, take 5
+    # to 9 ms instead of 10 to 33. In a loop of calls it would cost 3% (0.05 ms of 1.5), so blocks
+    # handed out within this time are left alone.
     _STALE = 0.05
 
     def __init__(self, limit: int = 512 << 20, smallest: int = 64 << 10, rest: int = 128 << 20):
